@@ -288,7 +288,7 @@ __device__ __forceinline__ int row_geometry(const Geom &g, uint32_t r, int32_t *
 // neighbours in state 1 comes out of the bit-sliced counter over the 2d
 // neighbour rows (d <= 3: at most 6), key cur + 2 * count as the byte body's.
 template <int D, class W>
-__device__ void packed_site_item(const LocalArgs &a, W *pk, int64_t chunk, int R, const uint32_t *tab) {
+__device__ void packed_site_item(const LocalArgs &a, W *pk, int64_t chunk, int R, const uint2 *tab) {
     const uint32_t L0 = (uint32_t)a.g.L[0];
     const uint32_t rows = row_count(a.g);
     const W full = L0 == 8 * sizeof(W) ? ~(W)0 : (((W)1 << L0) - 1);
@@ -362,7 +362,7 @@ __device__ long long packed_energy_rows(const LocalArgs &a, const W *pk, int lin
 // MU: the pass's direction (a compile-time constant, so the staple terms that
 // are row rotations and those that are other rows are fixed per variant).
 template <int D, int MU>
-__device__ void packed_link_item(const LocalArgs &a, uint32_t *pk, int64_t chunk, int R, const uint32_t *tab) {
+__device__ void packed_link_item(const LocalArgs &a, uint32_t *pk, int64_t chunk, int R, const uint2 *tab) {
     // (rows of at most 32 links)
     const uint32_t L0 = (uint32_t)a.g.L[0];
     const uint32_t rows = row_count(a.g);
@@ -741,7 +741,7 @@ template <int R, bool WORDS_ONLY>
 __global__ void __launch_bounds__(kEnsThreads, WORDS_ONLY ? 4 : 2) ensemble_kernel(EnsArgs e) {
     __shared__ LocalArgs sa;
     __shared__ unsigned long long s_ticket;
-    __shared__ uint32_t s_tab[16];  // a packed member's decision table (keys cur + 2 * count < 16)
+    __shared__ uint2 s_tab[kTableEntries + 1];  // a packed member's decision table (keys cur + 2 * count < 16)
     const unsigned long long n_items = (unsigned long long)e.n_items;
     const unsigned long long total = n_items * e.sweeps;
     if (threadIdx.x == 0) s_ticket = atomicAdd(&e.ls->ticket, 1ull);
@@ -785,7 +785,8 @@ __global__ void __launch_bounds__(kEnsThreads, WORDS_ONLY ? 4 : 2) ensemble_kern
         if (tk >= total) break;
         const int m = it.member, p = it.pass;
         PassFields pf;
-        uint32_t tv = 0;
+        uint2 tv = make_uint2(0, 0);
+        bool marked = false;
         const EnsMember &mem = e.members[m];
         if (threadIdx.x == 0) {
             const unsigned long long next = atomicAdd(&e.ls->ticket, 1ull);  // used after this item
@@ -795,7 +796,10 @@ __global__ void __launch_bounds__(kEnsThreads, WORDS_ONLY ? 4 : 2) ensemble_kern
             pf = pass_fields(e, m, p, r);
             const int k = (int)threadIdx.x - 32;
             const int nk = 2 + 4 * (mem.link ? mem.a.g.d - 1 : mem.a.g.d);  // keys of a q = 2 table
-            if (mem.pk && k < nk) tv = table_entry((mem.a.kernel == PLQ_HEATBATH ? pf.hb24 : pf.metro24)[k]);
+            uint32_t cut = 1;
+            if (mem.pk && k < nk) cut = (mem.a.kernel == PLQ_HEATBATH ? pf.hb24 : pf.metro24)[k];
+            tv = table_entry_marked(cut);
+            marked = __any_sync(0x0000ffffu, cut == 0);
         } else if (threadIdx.x == 64 && pending >= 0) {
             __threadfence();
             atomicAdd(&e.done[pending], (unsigned long long)pending_n);
@@ -808,6 +812,7 @@ __global__ void __launch_bounds__(kEnsThreads, WORDS_ONLY ? 4 : 2) ensemble_kern
         }
         __syncthreads();  // the wait is over, the previous item released, the arguments loaded
         if (threadIdx.x == 32) apply(pf, sa);
+        if (threadIdx.x == 32) s_tab[kTableEntries].x = marked ? 1u : 0u;
         if (threadIdx.x >= 32 && threadIdx.x < 48) s_tab[threadIdx.x - 32] = tv;
         // the next item's entry, loaded while this one runs
         const unsigned long long tk_next = s_ticket;

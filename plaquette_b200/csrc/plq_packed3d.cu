@@ -99,10 +99,21 @@ __global__ void __launch_bounds__(kPackedThreads) first_hash_kernel(uint4 *H, in
     }
 }
 
+// Bound by the integer pipe, with the first-hash stream (4 B per update) at two
+// thirds of the copy bandwidth.  512^3 Ising, 20 sweeps in one advance call, ms per
+// sweep Metropolis / heat bath: 0.1347 / 0.1395 with closed draws decided by
+// funnel-shifted differences at 32 registers; with open draws (plq_packed.cuh) 0.1266 /
+// 0.1266 at 32 registers (8 CTAs per SM), 0.122 / 0.119 at 48 (5: a word's first hashes
+// stay in flight), 0.121 / 0.121 at 64 (4).  16 CTAs' worth of words per SM with a
+// grid-stride loop; one CTA per 256 words was 4 % slower (the table staged more often).
 template <int D, bool HB, bool CACHED>
-__global__ void __launch_bounds__(kPackedThreads, 8) packed_pass_kernel(PackedPassArgs a) {
-    __shared__ uint32_t s_tab[16];
-    if (threadIdx.x < 16) s_tab[threadIdx.x] = threadIdx.x < (unsigned)a.n_keys ? table_entry(a.table[threadIdx.x]) : 0u;
+__global__ void __launch_bounds__(kPackedThreads, 5) packed_pass_kernel(PackedPassArgs a) {
+    __shared__ uint2 s_tab[kTableEntries + 1];
+    uint32_t cut = 1;
+    if (threadIdx.x < (unsigned)a.n_keys) cut = a.table[threadIdx.x];
+    if (threadIdx.x < kTableEntries) s_tab[threadIdx.x] = table_entry_marked(cut);
+    const bool marked = __syncthreads_or(cut == 0);
+    if (threadIdx.x == 0) s_tab[kTableEntries].x = marked ? 1u : 0u;
     __syncthreads();
     const uint32_t wpr = (uint32_t)a.L0 / 64;  // words per row
     const uint32_t rows = (uint32_t)(a.n_words / wpr);
@@ -116,13 +127,6 @@ __global__ void __launch_bounds__(kPackedThreads, 8) packed_pass_kernel(PackedPa
             y = r - z * (uint32_t)a.L1;
         } else {
             y = r;
-        }
-        uint4 hv[8];
-        if (CACHED) {  // this pass's 32 first hashes, issued before the neighbour loads
-            const uint4 *hp = static_cast<const uint4 *>(a.first_hash) +
-                              ((((int64_t)a.colour * ((a.n_words + 31) >> 5) + (g >> 5)) * 8) << 5) + (g & 31);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) hv[k] = __ldcs(hp + 32 * k);
         }
         const uint64_t *w = a.words;
         const uint32_t rb = r * wpr;
@@ -149,7 +153,9 @@ __global__ void __launch_bounds__(kPackedThreads, 8) packed_pass_kernel(PackedPa
         const uint32_t x0 = (uint32_t)((a.colour ^ y ^ z) & 1u);
         const uint32_t v0 = r * (uint32_t)a.L0 + 64u * wi + x0;  // keyed index of the word's first such site
         uint64_t flip;
-        if (CACHED) {
+        if (CACHED && !marked) {
+            const uint4 *hp = static_cast<const uint4 *>(a.first_hash) +
+                              ((((int64_t)a.colour * ((a.n_words + 31) >> 5) + (g >> 5)) * 8) << 5) + (g & 31);
             const uint64_t M = 0x5555555555555555ull;
             const uint64_t P = ((C >> x0) & M) | (((c0 >> x0) << 1) & ~M);
             const uint64_t Q = ((c1 >> x0) & M) | (((c2 >> x0) << 1) & ~M);
@@ -157,12 +163,11 @@ __global__ void __launch_bounds__(kPackedThreads, 8) packed_pass_kernel(PackedPa
             flip = 0;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const uint32_t h1[8] = {hv[2 * c].x,     hv[2 * c].y,     hv[2 * c].z,     hv[2 * c].w,
-                                        hv[2 * c + 1].x, hv[2 * c + 1].y, hv[2 * c + 1].z, hv[2 * c + 1].w};
+                const uint4 ha = __ldcs(hp + 64 * c), hb = __ldcs(hp + 64 * c + 32);
+                const uint32_t h1[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
                 flip |= (uint64_t)decide8_h1<HB>(key_word(P, Q, c), h1, sweep_mix, tb) << (16 * c);
             }
             if (HB) flip ^= P & M;  // new states -> flips
-            (void)v0;
         } else {
             flip = decide_row<uint64_t, 2, HB>(C >> x0, c0 >> x0, c1 >> x0, c2 >> x0, 32, v0, a.seed32, sweep_mix,
                                                s_tab);

@@ -206,10 +206,15 @@ PLQ_HD uint32_t lowbias32_head(uint32_t x) {
     v *= 0x846ca68bu;
     return v;
 }
-PLQ_HD uint32_t lowbias32_tail(uint32_t v) {
+// lowbias32_tail before its closing xorshift by 16.
+PLQ_HD uint32_t lowbias32_open(uint32_t v) {
     v *= 0x7feb352du;
     v ^= v >> 15;
     v *= 0x846ca68bu;
+    return v;
+}
+PLQ_HD uint32_t lowbias32_tail(uint32_t v) {
+    v = lowbias32_open(v);
     v ^= v >> 16;
     return v;
 }
