@@ -11,7 +11,7 @@
 //               axis-minor order (cluster.rs:44-62), placed by a device-wide
 //               exclusive scan (decoupled look-back) over agreeing bonds.
 //  2. labels -- lock-free union-find: every open bond unites its ends by
-//               hooking the larger root under the smaller with a CAS, first
+//               hooking the larger root under the smaller (an atomic minimum), first
 //               inside 64x64 tiles in shared memory (tile_hook_kernel), then
 //               for the bonds that leave a tile (boundary_hook_kernel); the
 //               relabel pass walks each site to its root (a short walk: sites
@@ -68,7 +68,8 @@ constexpr unsigned long long kDescAgg = 1ull, kDescPrefix = 2ull;
 struct ClusterArgs {
     uint8_t *state;
     uint8_t *bonds;
-    int32_t *parent;
+    int32_t *parent;      // union-find over the tile-local roots (flat over all sites after flatten_kernel)
+    uint16_t *local_root; // every site's tile-local root: by tile, then the place in the tile
     uint8_t *fresh;
     int32_t *rank;
     struct ChunkBase {     // stream relabel: per root_rank chunk, the state at the label draw of
@@ -330,17 +331,26 @@ __device__ __forceinline__ int32_t find_root(int32_t *parent, int32_t x, int cap
     return x;
 }
 
+// Unite the sets of a and b: the larger root is hooked under the smaller by an
+// atomic minimum on its parent.  Where that root was hooked in the meantime, its
+// parent becomes the smaller of the two all the same, and the link that gave way
+// (the old parent's) is united in turn: no attempt is repeated, so many lanes
+// hooking to one root do not wait for each other as they do on a CAS
+// (tile_hook_kernel on 2D Ising 4096^2 with 32-row blocks: 145 us with the CAS,
+// 131 with this).
 __device__ __forceinline__ void unite(int32_t *parent, int32_t a, int32_t b, int cap, Control *ctrl) {
     for (int it = 0;; ++it) {
         a = find_root(parent, a, cap, ctrl);
         b = find_root(parent, b, cap, ctrl);
         if (a == b) return;
-        if (a > b) {
+        if (a < b) {
             int32_t t = a;
             a = b;
             b = t;
         }
-        if (atomicCAS(&parent[b], b, a) == b) return;  // b was still a root: hooked under a
+        const int32_t old = atomicMin(&parent[a], b);
+        if (old == a) return;  // a was still a root
+        a = old;
         if (it > cap) {
             atomicOr(&ctrl->status, kStatusPassCap);
             return;
@@ -348,21 +358,109 @@ __device__ __forceinline__ void unite(int32_t *parent, int32_t a, int32_t b, int
     }
 }
 
-// ---- tile-local labelling: a CTA owns a T0 x T1 tile of (dims 0, 1), T0 and T1
-// the largest power-of-two divisors of L0, L1 capped at 64.  It unites the
-// open bonds inside the tile on a shared-memory parent array (same rule:
-// larger root under smaller, so each local root is the tile component's
-// minimum site; local and global index orders agree), then points every site
-// at its local root -- this is also the label init (cluster_prelude.wgsl:83-93)
-// of every site.  Only bonds that leave the tile go through the global
-// union-find (boundary_hook_kernel): ~2 / 64 of the bonds of a 2D lattice.
-constexpr int kTileMax = 64;
-constexpr int kTileSites = kTileMax * kTileMax;
+// ---- tile-local labelling.  A CTA labels a tile of TX x TY (x TZ, where the
+// lattice has a third direction) sites; its eight warps own blocks of 32
+// columns and walk their rows in order.  Within a row the runs of open +x bonds
+// come out of one ballot.  A run takes its label from the first open bond into
+// it from the row before (its y neighbour, else its z neighbour), so the walk
+// itself builds a forest one level deep without an atomic: at the 2D critical
+// point two runs in three find such a bond.  The bonds that remain -- a run's
+// further bonds to earlier rows, less those that repeat the lane before's pair,
+// and the bonds between blocks -- are united on the shared-memory parent array
+// (larger root under smaller, so each root is its component's minimum site:
+// local and global index orders agree).  What leaves the CTA is every site's
+// tile-local root, 16 bits at its place in the tile, and the global parent of
+// the roots themselves (the label init of cluster_prelude.wgsl:83-93): the
+// global union-find lives on the local roots alone, about one site in eight in
+// 2D at beta_c.  Bonds that leave the tile, the periodic ones among them, go
+// through it in boundary_hook_kernel; a relabel pass takes a tile per CTA, walks
+// once per local root and hands the labels to the sites in shared memory.
+//
+// Bound by issue: on the keyed stream about half of the instructions are the
+// two bond draws of a site.  2D Ising 4096^2 at beta_c in equilibrium, tile
+// kernel / relabel us a launch: 248 / 129 with a CAS union per +y bond (64 x 64
+// tiles) and a walk per site from a 32-bit parent; 120 / 37 so (the sweep
+// 0.41 -> 0.196 ms).  The block's 16 rows: 32 had fewer edges but its lists and
+// parents left 4 CTAs per SM (0.215 ms), 8 more boundary unions (0.217 ms).
+//
+// SMALL: fewer rows per block, for lattices that give the large tiles' CTAs to
+// less than two per SM (large_tiles): a block's rows are a serial chain.
+template <int D, bool SMALL>
+struct Tile {  // block (per warp): 32 x BY x BZ; tile: WX x WY x WZ blocks
+    static constexpr int BY = D == 1 ? 1 : D == 2 ? (SMALL ? 8 : 16) : (SMALL ? 2 : 4), BZ = D >= 3 ? (SMALL ? 2 : 4) : 1;
+    static constexpr int WX = D == 1 ? 8 : D == 2 ? 4 : (SMALL ? 1 : 2), WY = D == 1 ? 1 : D == 2 || !SMALL ? 2 : 4,
+                         WZ = D >= 3 ? 2 : 1;
+    static constexpr int TX = 32 * WX, TY = BY * WY, TZ = BZ * WZ;
+    static constexpr int kSites = TX * TY * TZ;
+    static constexpr int G = D == 2 ? 8 : BY;  // rows whose bonds are made together
+    static_assert(WX * WY * WZ * 32 == kThreads, "a warp per block");
+    static_assert(kSites <= 65536 && (BY * BZ) % G == 0 && BY * BZ <= 32, "16-bit local roots, 32 rows a block");
 
-__device__ __forceinline__ int tile_extent(int L) {
-    const int p2 = L & -L;  // largest power-of-two divisor
-    return p2 < kTileMax ? p2 : kTileMax;
+    int32_t L[3];
+    uint32_t plane, slab_sites;  // sites of an xy plane, of a slab (the tile's directions)
+    uint32_t t0, t1, t2;         // tiles along them
+    __host__ __device__ explicit Tile(const Geom &g) {
+        L[0] = g.L[0];
+        L[1] = D >= 2 ? g.L[1] : 1;
+        L[2] = D >= 3 ? g.L[2] : 1;
+        plane = (uint32_t)L[0] * (uint32_t)L[1];
+        slab_sites = plane * (uint32_t)L[2];
+        t0 = (uint32_t)(L[0] + TX - 1) / TX;
+        t1 = (uint32_t)(L[1] + TY - 1) / TY;
+        t2 = (uint32_t)(L[2] + TZ - 1) / TZ;
+    }
+    __host__ __device__ int64_t tiles(int64_t n_sites) const { return n_sites / slab_sites * t0 * t1 * t2; }
+    // First site of tile b, and its coordinates.
+    __device__ uint32_t origin(uint32_t b, int *x) const {
+        const uint32_t b1 = b / t0, b2 = b1 / t1, slab = D >= 3 ? b2 / t2 : b2;
+        x[0] = (int)(b - b1 * t0) * TX;
+        x[1] = (int)(b1 - b2 * t1) * TY;
+        x[2] = D >= 3 ? (int)(b2 - slab * t2) * TZ : 0;
+        return slab * slab_sites + (uint32_t)x[2] * plane + (uint32_t)x[1] * (uint32_t)L[0] + (uint32_t)x[0];
+    }
+    // The site at place li of the tile whose first site is s0.
+    __device__ uint32_t site(uint32_t s0, uint32_t li) const {
+        uint32_t s = s0 + li % TX;
+        if (D >= 2) s += li / TX % TY * (uint32_t)L[0];
+        if (D >= 3) s += li / (TX * TY) * plane;
+        return s;
+    }
+    // Whether place li of the tile at x is in the lattice (tiles overhang).
+    __device__ bool inside(const int *x, uint32_t li) const {
+        return x[0] + (int)(li % TX) < L[0] && (D < 2 || x[1] + (int)(li / TX % TY) < L[1]) &&
+               (D < 3 || x[2] + (int)(li / (TX * TY)) < L[2]);
+    }
+    // The tile-local root of the site at coordinates x (x[2] and up: its slab), as a site.
+    __device__ uint32_t local_root(const uint16_t *roots, uint32_t s, const int32_t *x) const {
+        const uint32_t xx = (uint32_t)x[0], y = D >= 2 ? (uint32_t)x[1] : 0u, z = D >= 3 ? (uint32_t)x[2] : 0u;
+        const uint32_t slab = D > 3 ? s / slab_sites : 0u;
+        const uint32_t tile = ((slab * t2 + z / TZ) * t1 + y / TY) * t0 + xx / TX;
+        const uint32_t li = ((z % TZ) * TY + y % TY) * TX + xx % TX;
+        const uint32_t r = roots[(size_t)tile * kSites + li];
+        return s - (xx % TX) - (y % TY) * (uint32_t)L[0] - (z % TZ) * plane + site(0, r);
+    }
+};
+
+// Whether the large tiles give every SM two CTAs.
+template <int D>
+bool large_tiles(const Geom &g, int sm_count) {
+    return D >= 2 && Tile<D, false>(g).tiles(g.n_sites) >= 2 * (int64_t)sm_count;
 }
+
+// The keyed bond draw of one sweep as an open-draw comparison (plq_packed.cuh):
+// k < kp24 with k the 24-bit draw <=> (v ^ X) <= T, v the draw before its
+// closing xorshift.
+// (kp24 = 0, no bond opens, has no T: some() says so, once for a group of draws.)
+struct BondCut {
+    uint32_t seed, mix, T, X;
+    __device__ __forceinline__ explicit BondCut(const ClusterArgs &a)
+        : seed(a.seed32 ^ kBondKey), mix(keyed_mix(a.sweep32)), T((a.kp24 << 8) - 1u),
+          X(((a.kp24 << 8) - 1u) >> 16) {}
+    __device__ __forceinline__ bool open(uint32_t bond) const {
+        return (lowbias32_open(lowbias32_head(seed ^ bond) ^ mix) ^ X) <= T;
+    }
+    static __device__ __forceinline__ bool some(const ClusterArgs &a) { return a.kp24 != 0; }
+};
 
 __device__ __forceinline__ int lfind(int32_t *p, int32_t x, int cap, Control *ctrl) {
     int32_t px = p[x];
@@ -386,12 +484,14 @@ __device__ __forceinline__ void lunite(int32_t *p, int32_t a, int32_t b, int cap
         a = lfind(p, a, cap, ctrl);
         b = lfind(p, b, cap, ctrl);
         if (a == b) return;
-        if (a > b) {
+        if (a < b) {
             const int32_t t = a;
             a = b;
             b = t;
         }
-        if (atomicCAS(&p[b], b, a) == b) return;
+        const int32_t old = atomicMin(&p[a], b);  // as unite
+        if (old == a) return;
+        a = old;
         if (it > cap) {
             atomicOr(&ctrl->status, kStatusPassCap);
             return;
@@ -399,148 +499,278 @@ __device__ __forceinline__ void lunite(int32_t *p, int32_t a, int32_t b, int cap
     }
 }
 
-template <int D, bool KEYED>
-__global__ void __launch_bounds__(kThreads) tile_hook_kernel(ClusterArgs a) {
-    __shared__ int32_t p[kTileSites];
-    __shared__ uint8_t bs[kTileSites];  // the tile's bond bytes
-    const int L0 = a.g.L[0], L1 = D >= 2 ? a.g.L[1] : 1;
-    const int T0 = tile_extent(L0), T1 = D >= 2 ? tile_extent(L1) : 1;
-    const int T = T0 * T1;
-    const int tiles0 = L0 / T0, tiles1 = L1 / T1;
-    // tile origin: (tx * T0, ty * T1, slab) with slab the index over dims >= 2
-    const int64_t bid = blockIdx.x;
-    const int tx = (int)(bid % tiles0);
-    const int64_t r1 = bid / tiles0;
-    const int ty = (int)(r1 % tiles1);
-    const int64_t slab = r1 / tiles1;
-    const int64_t base = slab * (int64_t)L0 * L1 + (int64_t)ty * T1 * L0 + (int64_t)tx * T0;
-    const int cap = a.cap < kTileSites + 64 ? a.cap : kTileSites + 64;
-    // T0 is a power of two: local index li = yl * T0 + xl splits by shift and mask (a runtime
-    // division would cost ~20 instructions, several times per site)
-    const int sh0 = __ffs(T0) - 1, m0 = T0 - 1;
-    // x runs first: a warp holds 32 consecutive sites; each site points straight at
-    // the start of its run of open +x bonds (the run's minimum), found with one ballot
-    const int lane = threadIdx.x & 31;
-    const int rounds = (T + (int)blockDim.x - 1) / (int)blockDim.x;
-    for (int k = 0; k < rounds; ++k) {
-        const int li = k * (int)blockDim.x + (int)threadIdx.x;
-        const bool valid = li < T;
-        const int xl = li & m0;
-        uint32_t own = 0;
-        if (valid) {
-            const int64_t s = base + xl + (int64_t)(li >> sh0) * L0;
-            if (KEYED) {
-                // +x and +y bonds from the spins and the keyed draws (the bonds along
-                // dims >= 2 all leave the tile: boundary_hook_kernel evaluates them)
-                const int xg = tx * T0 + xl;
-                own = keyed_bond<D>(a, s, 0, xg + 1 < L0 ? s + 1 : s + 1 - L0) ? 1u : 0u;
-                if (D >= 2) {
-                    const int yg = ty * T1 + (li >> sh0);
-                    own |= keyed_bond<D>(a, s, 1, yg + 1 < L1 ? s + L0 : s - (int64_t)(L1 - 1) * L0) ? 2u : 0u;
-                }
-            } else {
-                own = a.bonds[s];
-            }
-        }
-        if (valid) bs[li] = (uint8_t)own;
-        // the bond into this site from its -x neighbour (lane - 1), inside this warp's segment
-        const uint32_t from_left = __shfl_up_sync(0xffffffffu, own, 1);
-        const bool joined = valid && lane > 0 && xl > 0 && (from_left & 1u) != 0;
-        const unsigned starts = __ballot_sync(0xffffffffu, !joined);
-        const int start = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));
-        if (valid) p[li] = li - lane + start;
-    }
-    __syncthreads();
-    // the remaining bonds inside the tile: +x across a warp segment or around the row, and +y.
-    // (Skipping a +y bond that the x-1 bonds already imply saves 16 % of these unions at
-    // criticality but measured slower: the extra shared-memory reads cost more.)
-    for (int li = threadIdx.x; li < T; li += blockDim.x) {
-        const int xl = li & m0, yl = li >> sh0;
-        const uint32_t b = bs[li];
-        if (b & 1u) {
-            if (xl + 1 < T0) {
-                if ((li & 31) == 31) lunite(p, li, li + 1, cap, a.ctrl);
-            } else if (T0 == L0) {
-                lunite(p, li, li - (T0 - 1), cap, a.ctrl);
-            }
-        }
-        if (D >= 2 && (b & 2u)) {  // +y inside the tile
-            if (yl + 1 < T1) lunite(p, li, li + T0, cap, a.ctrl);
-            else if (T1 == L1) lunite(p, li, li - T0 * (T1 - 1), cap, a.ctrl);
-        }
-    }
-    __syncthreads();
-    // The forest is final: each site walks to its local root (read-only; trees at β_c are
-    // about 2.3 deep on average, at most ~10, so this beats block-wide pointer-jumping rounds)
-    // and points at it.
-    for (int li = threadIdx.x; li < T; li += blockDim.x) {
-        int32_t r = li;
-        for (int it = 0; p[r] != r && it < kTileSites; ++it) r = p[r];
-        const int64_t s = base + (li & m0) + (int64_t)(li >> sh0) * L0;
-        a.parent[s] = (int32_t)(base + (r & m0) + (int64_t)(r >> sh0) * L0);
-    }
+// Unite the ends of an edge between blocks, one per lane (open: this lane has
+// one); a lane whose ends read as the lane before's pair leaves it to that lane.
+__device__ __forceinline__ void edge_unite(int32_t *p, bool open, int32_t u, int32_t v, int cap, Control *ctrl) {
+    const int32_t pu = open ? p[u] : -1, pv = open ? p[v] : -1;
+    const int32_t qu = __shfl_up_sync(0xffffffffu, pu, 1), qv = __shfl_up_sync(0xffffffffu, pv, 1);
+    const bool repeat = (threadIdx.x & 31u) > 0 && qu == pu && qv == pv;
+    if (open && !repeat && pu != pv) lunite(p, pu, pv, cap, ctrl);
 }
 
-// Global unions for the open bonds that leave their tile: +x bonds of the
-// tile's last column (when tiles split the rows), +y bonds of its last row
-// (when tiles split dim 1), and every bond along dims >= 2.  Thread t of the
-// grid takes candidate site t of each family in turn.
-template <int D, bool KEYED>
-__global__ void __launch_bounds__(kThreads) boundary_hook_kernel(ClusterArgs a) {
-    const int64_t n = a.g.n_sites;
-    const int L0 = a.g.L[0], L1 = D >= 2 ? a.g.L[1] : 1;
-    const int T0 = tile_extent(L0), T1 = D >= 2 ? tile_extent(L1) : 1;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    // the two families in one index space, so a thread makes at most one union of them:
-    // candidates c < nx are sites with x = k*T0 + T0-1 (n / T0 of them), the rest the sites of
-    // rows with y = k*T1 + T1-1 (n / T1)
-    const int64_t nx = T0 < L0 ? n / T0 : 0;
-    const int64_t ny = D >= 2 && T1 < L1 ? n / T1 : 0;
-    const int64_t per_row = L0;
-    for (int64_t c = t0; c < nx + ny; c += stride) {
-        int64_t s;
-        int mu;
-        if (c < nx) {
-            s = c * T0 + (T0 - 1);
-            mu = 0;
+template <int D, bool SMALL, bool KEYED>
+__global__ void __launch_bounds__(kThreads, D == 2 && !SMALL ? 5 : 1) tile_hook_kernel(ClusterArgs a) {
+    using T = Tile<D, SMALL>;
+    constexpr int BY = T::BY, BZ = T::BZ, TX = T::TX, TY = T::TY, TZ = T::TZ, G = T::G;
+    constexpr int kBlock = 32 * BY * BZ, kFurther = D >= 3 ? 2 * kBlock : D == 2 ? kBlock : 1;
+    __shared__ int32_t p[T::kSites];
+    __shared__ uint16_t s_further[kThreads / 32][kFurther];
+    const T t(a.g);
+    const int L0 = t.L[0], L1 = t.L[1], L2 = t.L[2];
+    int xt[3];
+    const uint32_t s_tile = t.origin(blockIdx.x, xt);
+    const int cap = a.cap < T::kSites + 64 ? a.cap : T::kSites + 64;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int wx = wid % T::WX, wy = (wid / T::WX) % T::WY, wz = wid / (T::WX * T::WY);
+    const int lx = 32 * wx + lane, x = xt[0] + lx;
+    const int ly0 = wy * BY, y0 = xt[1] + ly0, lz0 = wz * BZ, z0 = xt[2] + lz0;
+    const bool in_x = x < L0;
+    const uint32_t plane = t.plane;
+    const uint32_t s00 = s_tile + (uint32_t)lz0 * plane + (uint32_t)(ly0 * L0 + lx);
+    const int li00 = (lz0 * TY + ly0) * TX + lx;
+    const uint32_t le = 0xffffffffu >> (31 - lane);
+    const BondCut cut(a);
+    const bool x_in_tile = x + 1 < L0 && lx + 1 < TX;  // the +x neighbour is in the tile
+
+    // ---- the block's rows in order: labels from the row before and the plane before
+    // further bonds to the row before (the site's place) or the plane before (| kToPlane), listed per
+    // block: about one site in ten has one, and a list keeps whole warps busy uniting them
+    constexpr uint32_t kToPlane = 0x8000u;
+    static_assert(D < 3 || T::kSites <= 0x8000, "a bit beside the place");
+    uint16_t *further = s_further[wid];
+    int n_further = 0;
+    uint32_t mine = 0;  // rows whose label is this lane's own site
+    auto list = [&](bool mine, uint32_t entry) {
+        const unsigned m = __ballot_sync(0xffffffffu, mine);
+        if (mine) further[n_further + __popc(m & (le >> 1))] = (uint16_t)entry;
+        n_further += __popc(m);
+    };
+    uint32_t edge_x = 0;              // lane 31: rows with an open bond to the next block
+    uint32_t edge_y = 0, edge_z = 0;  // planes / rows with an open bond to the next block
+    int32_t lab_plane[D >= 3 ? BY : 1] = {};
+    uint32_t open_plane = 0;  // bit y: the plane before's +z bond
+    int32_t lab_up = 0;
+    bool open_up = false;
+#pragma unroll 1
+    for (int g = 0; g < BY * BZ / G; ++g) {
+        const int jz = D >= 3 ? g : 0, yg = D >= 3 ? 0 : g * G;
+        if ((D >= 3 && z0 + jz >= L2) || y0 + yg >= L1) break;
+        const uint32_t sg = s00 + (uint32_t)jz * plane + (uint32_t)(yg * L0);
+        const bool z_in_tile = D >= 3 && z0 + jz + 1 < L2 && lz0 + jz + 1 < TZ;
+        // the bonds of G rows, their loads in flight together
+        uint32_t bx = 0, by = 0, bz = 0;
+        if (KEYED) {
+            uint32_t c[G + 1], cr[G], cz[G];
+#pragma unroll
+            for (int k = 0; k <= G; ++k) c[k] = in_x && y0 + yg + k < L1 ? a.state[sg + (uint32_t)(k * L0)] : 0u;
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+                cr[k] = lane == 31 && x_in_tile && y0 + yg + k < L1 ? a.state[sg + (uint32_t)(k * L0) + 1u] : 0u;
+                cz[k] = D >= 3 && z_in_tile && in_x && y0 + yg + k < L1 ? a.state[sg + (uint32_t)(k * L0) + plane] : 0u;
+            }
+            // every lane draws every bond (a branch around a draw that one lane in seven skips
+            // costs more than it saves); what is not a bond of the tile is masked at the end
+            uint32_t ax = 0, ay = 0, az = 0;
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+                const uint32_t bond = (sg + (uint32_t)(k * L0)) * (uint32_t)D;
+                const uint32_t down = __shfl_down_sync(0xffffffffu, c[k], 1);
+                const uint32_t right = lane == 31 ? cr[k] : down;
+                if ((c[k] == right) & cut.open(bond)) bx |= 1u << k;
+                if (D >= 2 && ((c[k] == c[k + 1]) & cut.open(bond + 1u))) by |= 1u << k;
+                if (D >= 3 && ((c[k] == cz[k]) & cut.open(bond + 2u))) bz |= 1u << k;
+            }
+            if (BondCut::some(a)) {
+                const int rows = min(G, L1 - (y0 + yg));  // rows of the group in the lattice
+                const uint32_t in_rows = (1u << rows) - 1u;
+                if (x_in_tile) ax = in_rows;
+                if (in_x && z_in_tile) az = in_rows;
+                // a row's +y neighbour: the row after it in the lattice and the tile
+                const int rows_y = min(min(G, L1 - 1 - (y0 + yg)), TY - 1 - (ly0 + yg));
+                if (in_x && D >= 2) ay = (1u << rows_y) - 1u;
+            }
+            bx &= ax;
+            by &= ay;
+            bz &= az;
         } else {
-            const int64_t cy = c - nx;
-            const int64_t row = fdiv((uint32_t)cy, a.g.dm[0], a.g.dl[0]);  // index among the selected rows
-            s = (row * T1 + (T1 - 1)) * per_row + (cy - row * per_row);
-            mu = 1;
+            uint32_t own[G];
+#pragma unroll
+            for (int k = 0; k < G; ++k) own[k] = in_x && y0 + yg + k < L1 ? a.bonds[sg + (uint32_t)(k * L0)] : 0u;
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+                if (x_in_tile) bx |= (own[k] & 1u) << k;
+                if (y0 + yg + k + 1 < L1 && ly0 + yg + k + 1 < TY) by |= ((own[k] >> 1) & 1u) << k;
+                if (z_in_tile) bz |= ((own[k] >> 2) & 1u) << k;
+            }
         }
-        if (!KEYED && !((a.bonds[s] >> mu) & 1u)) continue;
-        int32_t x[D];
-        site_coords<D>(a.g, s, x);
-        // compile-time directions keep the coordinates in registers
-        const int64_t nb = mu == 0 ? nbr_plus(a.g, s, x, 0) : nbr_plus(a.g, s, x, D >= 2 ? 1 : 0);
-        if (KEYED && !keyed_bond<D>(a, s, mu, nb)) continue;
-        unite(a.parent, (int32_t)s, (int32_t)nb, a.cap, a.ctrl);
+        if (D >= 3) {
+            open_up = false;
+            if (jz == BZ - 1) edge_z = bz;
+        }
+        if (lane == 31) edge_x |= bx << (g * G);
+        // the labels of the G rows, one after the other
+#pragma unroll
+        for (int k = 0; k < G; ++k) {
+            if (y0 + yg + k >= L1) break;
+            // the run of this lane: lanes [st, next start)
+            const uint32_t starts = ~(__ballot_sync(0xffffffffu, (bx >> k) & 1u) << 1);
+            const int st = 31 - __clz(starts & le);
+            const uint32_t later = starts & ~le;
+            const uint32_t run = ((later & (0u - later)) - 1u) & (0xffffffffu << st);
+            const int li = li00 + (jz * TY + yg + k) * TX;
+            int32_t label = li - lane + st;
+            const uint32_t up = __ballot_sync(0xffffffffu, open_up) & run;
+            const int32_t from_up = __shfl_sync(0xffffffffu, lab_up, (__ffs(up) - 1) & 31);
+            if (up) label = from_up;
+            if (D >= 3) {
+                const bool oz = (open_plane >> k) & 1u;
+                const int32_t lab_z = lab_plane[k];
+                const uint32_t uz = __ballot_sync(0xffffffffu, oz) & run;
+                const int32_t from_z = __shfl_sync(0xffffffffu, lab_z, (__ffs(uz) - 1) & 31);
+                if (!up && uz) label = from_z;
+                const int32_t before = __shfl_up_sync(0xffffffffu, lab_z, 1);
+                const bool repeat = before == lab_z && ((uz << 1) >> lane) & 1u;
+                list(oz && !repeat && lab_z != label, (uint32_t)li | kToPlane);
+                lab_plane[k] = label;
+            }
+            {
+                const int32_t before = __shfl_up_sync(0xffffffffu, lab_up, 1);
+                const bool repeat = before == lab_up && ((up << 1) >> lane) & 1u;
+                if (D >= 2) list(open_up && !repeat && lab_up != label, (uint32_t)li);
+            }
+            p[li] = label;
+            if (label == li) mine |= 1u << (g * G + k);
+            lab_up = label;
+            open_up = (by >> k) & 1u;
+        }
+        if (yg + G == BY && y0 + BY < L1 && (by >> (G - 1)) & 1u) edge_y |= 1u << jz;
+        open_plane = bz;
+    }
+    __syncthreads();
+
+    // ---- the remaining bonds of the tile
+    for (int i = lane; i < n_further; i += 32) {
+        const uint32_t e = further[i];
+        const int li = D >= 3 ? (int)(e & ~kToPlane) : (int)e;
+        lunite(p, li, li - (D >= 3 && (e & kToPlane) ? TX * TY : TX), cap, a.ctrl);
+    }
+    __syncwarp();
+    if (T::WX > 1) {  // bonds between blocks: lane l takes row l of the block's last column, its own column's last rows
+        const uint32_t rows = __shfl_sync(0xffffffffu, edge_x, 31);
+        const int li = li00 - lane + 31 + (lane / BY * TY + lane % BY) * TX;
+        const bool open = lane < BY * BZ && ((rows >> lane) & 1u);
+        edge_unite(p, open, li, li + 1, cap, a.ctrl);
+    }
+    if (D >= 2) {
+#pragma unroll
+        for (int jz = 0; jz < BZ; ++jz) {
+            const int li = li00 + (jz * TY + BY - 1) * TX;
+            edge_unite(p, (edge_y >> jz) & 1u, li, li + TX, cap, a.ctrl);
+        }
     }
     if (D >= 3) {
-        for (int64_t s = t0; s < n; s += stride) {
-            uint8_t b = 0;
-            int32_t x[D];
-            if (KEYED) {
-                site_coords<D>(a.g, s, x);
 #pragma unroll
-                for (int mu = 2; mu < D; ++mu)
-                    if (keyed_bond<D>(a, s, mu, nbr_plus(a.g, s, x, mu))) b |= (uint8_t)(1u << (mu - 2));
-            } else {
-                b = (uint8_t)(a.bonds[s] >> 2);
-                if (!b) continue;
-                site_coords<D>(a.g, s, x);
-            }
-#pragma unroll
-            for (int mu = 2; mu < D; ++mu)
-                if ((b >> (mu - 2)) & 1u) unite(a.parent, (int32_t)s, (int32_t)nbr_plus(a.g, s, x, mu), a.cap, a.ctrl);
+        for (int jy = 0; jy < BY; ++jy) {
+            const int li = li00 + ((BZ - 1) * TY + jy) * TX;
+            edge_unite(p, (edge_z >> jy) & 1u, li, li + TX * TY, cap, a.ctrl);
+        }
+    }
+    __syncthreads();
+
+    // ---- the forest is final.  The labels the rows were given (the sites whose label was their
+    // own: mine) are pointed at their roots, which leaves every site two steps from its root.
+    for (uint32_t m = mine; m; m &= m - 1u) {
+        const int j = __ffs(m) - 1;
+        const int li = li00 + (j / BY * TY + j % BY) * TX;
+        const int32_t r = lfind(p, li, cap, a.ctrl);
+        if (r != li) p[li] = r;
+    }
+    __syncthreads();
+    if (!in_x) return;
+    uint16_t *roots = a.local_root + (size_t)blockIdx.x * T::kSites;
+#pragma unroll 1
+    for (int jz = 0; jz < BZ; ++jz) {
+        if (D >= 3 && z0 + jz >= L2) break;
+#pragma unroll 8
+        for (int jy = 0; jy < BY; ++jy) {
+            if (y0 + jy >= L1) break;
+            const int li = li00 + (jz * TY + jy) * TX;
+            const int32_t r = p[p[li]];
+            const uint32_t s = s00 + (uint32_t)jz * plane + (uint32_t)(jy * L0);
+            roots[li] = (uint16_t)r;
+            if (r == li) a.parent[s] = (int32_t)s;
+            if (!KEYED) a.fresh[s] = r == li ? 1 : 0;  // root_rank_kernel's candidates, in site order
         }
     }
 }
 
-// Read-only find for the relabel pass: a compressing find could overwrite a
-// site another thread has just set to its root with a non-root ancestor.
+// Global unions for the open bonds that leave their tile: of the tiles' last
+// columns, last rows and last planes (three families of candidate sites in one
+// index space), and every bond along the directions past the tile's.  A lane
+// whose ends' local roots are the lane before's leaves the union to that lane:
+// along a tile edge a large cluster meets another at many sites.
+template <int D, bool SMALL, bool KEYED>
+__global__ void __launch_bounds__(kThreads) boundary_hook_kernel(ClusterArgs a) {
+    using T = Tile<D, SMALL>;
+    const T t(a.g);
+    const int64_t n = a.g.n_sites;
+    const uint32_t L0 = (uint32_t)t.L[0], L1 = (uint32_t)t.L[1], L2 = (uint32_t)t.L[2];
+    const uint32_t rows = (uint32_t)(n / L0), planes = rows / L1;  // planes: over every direction past 1
+    const int64_t nx = (int64_t)t.t0 * rows;
+    const int64_t ny = D >= 2 ? (int64_t)t.t1 * L0 * planes : 0;
+    const int64_t nz = D >= 3 ? (int64_t)t.t2 * t.plane * (planes / L2) : 0;
+    const int64_t candidates = nx + ny + nz, all = candidates + (D > 3 ? (int64_t)(D - 3) * n : 0);
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31;
+    // whole warps per trip: the comparison with the lane before is warp-wide
+    for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); c0 < all; c0 += stride) {
+        const int64_t c = c0 + lane;
+        int64_t s = 0;
+        int mu = 0;
+        if (c < nx) {
+            const uint32_t row = (uint32_t)c / t.t0, k = (uint32_t)c - row * t.t0;
+            s = (int64_t)row * L0 + min((k + 1u) * (uint32_t)T::TX, L0) - 1u;
+        } else if (c < nx + ny) {
+            const uint32_t cy = (uint32_t)(c - nx), r = cy / L0, xx = cy - r * L0, pl = r / t.t1, k = r - pl * t.t1;
+            s = ((int64_t)pl * L1 + min((k + 1u) * (uint32_t)T::TY, L1) - 1u) * L0 + xx;
+            mu = 1;
+        } else if (c < candidates) {
+            const uint32_t cz = (uint32_t)(c - nx - ny), r = cz / t.plane, xy = cz - r * t.plane, b = r / t.t2,
+                           k = r - b * t.t2;
+            s = ((int64_t)b * L2 + min((k + 1u) * (uint32_t)T::TZ, L2) - 1u) * t.plane + xy;
+            mu = 2;
+        } else if (c < all) {
+            const int64_t e = c - candidates;
+            mu = 3 + (int)(e / n);
+            s = e - (int64_t)(mu - 3) * n;
+        }
+        bool open = c < all;
+        if (!KEYED && open) open = (a.bonds[s] >> mu) & 1u;
+        int32_t pa = -1, pb = -1;
+        if (open) {
+            int32_t x[D];
+            site_coords<D>(a.g, s, x);
+            int64_t nb = 0;  // compile-time directions keep the coordinates in registers
+#pragma unroll
+            for (int m = 0; m < D; ++m)
+                if (m == mu) nb = nbr_plus(a.g, s, x, m);
+            if (KEYED) open = keyed_bond<D>(a, s, mu, nb);
+            if (open) {
+                pa = (int32_t)t.local_root(a.local_root, (uint32_t)s, x);
+#pragma unroll
+                for (int m = 0; m < D; ++m)
+                    if (m == mu) x[m] = x[m] + 1 < a.g.L[m] ? x[m] + 1 : 0;
+                pb = (int32_t)t.local_root(a.local_root, (uint32_t)nb, x);
+            }
+        }
+        const int32_t qa = __shfl_up_sync(0xffffffffu, pa, 1), qb = __shfl_up_sync(0xffffffffu, pb, 1);
+        const bool repeat = lane > 0 && qa == pa && qb == pb;
+        if (open && !repeat && pa != pb) unite(a.parent, pa, pb, a.cap, a.ctrl);
+    }
+}
+
+// Read-only find for the passes after the unions: a compressing find could
+// overwrite a root another thread has just stored with a non-root ancestor.
 __device__ __forceinline__ int32_t find_root_ro(const int32_t *parent, int32_t x, int cap, Control *ctrl) {
     int32_t p = ld_relaxed32(&parent[x]);
     int it = 0;
@@ -555,65 +785,122 @@ __device__ __forceinline__ int32_t find_root_ro(const int32_t *parent, int32_t x
     return x;
 }
 
-// Sites a thread resolves at once (stride apart): the loads of all of them
-// are issued before any is used, so their latencies overlap.
-constexpr int kRootBatch = 4;
-
-// The roots of sites s0, s0 + stride, ... after the boundary unions; also
-// stores them, which leaves the parent array flat (every site holding its
-// root) for the readers after the sweep.  tile_hook left every site pointing
-// at its local root, and the boundary unions only re-point roots (or halve
-// paths onto local roots), so the walk from a site's parent is short: at
-// beta_c about 7 % of the local roots end up under another root, a few levels
-// deep at most.  Every value stored is a final root, so concurrent walks stay
-// correct.
-__device__ __forceinline__ void take_roots(const ClusterArgs &a, int64_t s0, int64_t stride, int64_t n,
-                                           int32_t *root) {
-    int32_t p[kRootBatch], q[kRootBatch];
+// A relabel pass over one tile.  The tile's local roots are gathered into a list
+// in shared memory; each walks to its cluster's root once (and stores it, so
+// walks through it end there), and of_root(root) gives the value of its sites;
+// then out takes the sites of each row four at a time.  Bound by the latency of the
+// walks, hence the list: full warps of walks instead of one lane in eight.
+template <class T, class V, class F, class O>
+__device__ __forceinline__ void tile_relabel(const ClusterArgs &a, F of_root, O out) {
+    __shared__ __align__(16) uint16_t s_root[T::kSites];
+    __shared__ uint16_t s_list[T::kSites];
+    __shared__ V s_value[T::kSites];
+    __shared__ int s_n;
+    const T t(a.g);
+    int xt[3];
+    const uint32_t s_tile = t.origin(blockIdx.x, xt);
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    const uint4 *src = reinterpret_cast<const uint4 *>(a.local_root + (size_t)blockIdx.x * T::kSites);
+#pragma unroll(T::kSites / 8 / kThreads > 4 ? 4 : 1)
+    for (uint32_t i = threadIdx.x; i < T::kSites / 8; i += kThreads) {
+        const uint4 v = src[i];
+        reinterpret_cast<uint4 *>(s_root)[i] = v;
+        const uint32_t own = 8u * i | (8u * i + 1u) << 16;  // places 8i, 8i + 1; the next pairs step by 2
+        const uint32_t d[4] = {v.x ^ own, v.y ^ (own + 0x00020002u), v.z ^ (own + 0x00040004u),
+                               v.w ^ (own + 0x00060006u)};
+        uint32_t mine = 0;
 #pragma unroll
-    for (int k = 0; k < kRootBatch; ++k) {
-        const int64_t s = s0 + k * stride;
-        p[k] = s < n ? a.parent[s] : 0;  // only this thread writes parent[s] here
+        for (int k = 0; k < 4; ++k) {
+            if ((d[k] & 0xFFFFu) == 0) mine |= 1u << (2 * k);
+            if ((d[k] >> 16) == 0) mine |= 2u << (2 * k);
+        }
+        if (mine) {
+            int at = atomicAdd(&s_n, __popc(mine));
+            for (; mine; mine &= mine - 1u) s_list[at++] = (uint16_t)(8u * i + (uint32_t)__ffs(mine) - 1u);
+        }
     }
+    __syncthreads();
+    const int n = s_n;
+    for (int i0 = threadIdx.x; i0 < n; i0 += 4 * kThreads) {
+        uint32_t li[4];
+        int32_t s[4], up[4];
 #pragma unroll
-    for (int k = 0; k < kRootBatch; ++k) q[k] = s0 + k * stride < n ? ld_relaxed32(&a.parent[p[k]]) : 0;
+        for (int k = 0; k < 4; ++k) {  // the first steps of four walks in flight together
+            const int i = i0 + k * kThreads;
+            li[k] = i < n ? s_list[i] : 0u;
+            s[k] = i < n && t.inside(xt, li[k]) ? (int32_t)t.site(s_tile, li[k]) : -1;  // (an overhanging place holds anything)
+            up[k] = s[k] >= 0 ? ld_relaxed32(&a.parent[s[k]]) : -1;
+        }
 #pragma unroll
-    for (int k = 0; k < kRootBatch; ++k) {
-        const int64_t s = s0 + k * stride;
-        root[k] = 0;
-        if (s >= n) continue;
-        const int32_t r = q[k] == p[k] ? p[k] : find_root_ro(a.parent, q[k], a.cap, a.ctrl);
-        if (r != p[k]) a.parent[s] = r;
-        root[k] = r;
+        for (int k = 0; k < 4; ++k) {
+            if (s[k] < 0) continue;
+            int32_t root = s[k];
+            if (up[k] != s[k]) {
+                root = find_root_ro(a.parent, up[k], a.cap, a.ctrl);
+                if (root != up[k]) a.parent[s[k]] = root;
+            }
+            s_value[li[k]] = of_root(root);
+        }
+    }
+    __syncthreads();
+    // four sites of a row per thread
+    for (uint32_t li = 4u * threadIdx.x; li < T::kSites; li += 4u * kThreads) {
+        if (!t.inside(xt, li)) continue;
+        const uint2 r2 = *reinterpret_cast<const uint2 *>(s_root + li);
+        constexpr uint32_t kIn = T::kSites - 1;  // (places past the row's end hold anything)
+        static_assert((T::kSites & (T::kSites - 1)) == 0, "a power of two");
+        const uint32_t r[4] = {r2.x & kIn, (r2.x >> 16) & kIn, r2.y & kIn, (r2.y >> 16) & kIn};
+        const int last = t.L[0] - xt[0] - (int)(li % T::TX);  // sites left in the row
+        out(t.site(s_tile, li), last < 4 ? last : 4, r, s_value, t, s_tile);
     }
 }
 
-// ----------------------------------------------------------- 3. relabel
-// keyed (cluster_relabel.wgsl:72-89), every cluster
-__global__ void relabel_keyed_kernel(ClusterArgs a) {
-    const int64_t n = a.g.n_sites;
-    const uint32_t q = (uint32_t)a.q;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t s0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s0 < n; s0 += stride * kRootBatch) {
-        int32_t roots[kRootBatch];
-        take_roots(a, s0, stride, n, roots);
-#pragma unroll
-        for (int k = 0; k < kRootBatch; ++k) {
-            const int64_t s = s0 + k * stride;
-            if (s >= n) continue;
-            const uint32_t root = (uint32_t)roots[k];
-            float u = __fmul_rn((float)keyed24(a.seed32 ^ kRootSalt, root, a.sweep32), 5.9604644775390625e-8f);
-            if (a.relabel == PLQ_RELABEL_FORCED) {
-                uint32_t step = __float2uint_rz(__fmul_rn(u, (float)(q - 1u)));
-                if (step >= q - 1u) step = q - 2u;
-                a.state[s] = (uint8_t)((a.state[s] + 1u + step) % q);
-            } else {
-                uint32_t draw = __float2uint_rz(__fmul_rn(u, (float)q));
-                if (draw >= q) draw = q - 1u;
-                a.state[s] = (uint8_t)draw;
-            }
-        }
+// The values of up to four sites of a row into a byte array.
+__device__ __forceinline__ void store_row(uint8_t *state, uint32_t s, int count, const uint8_t *v) {
+    if (count == 4 && (s & 3u) == 0) {
+        *reinterpret_cast<uchar4 *>(state + s) = make_uchar4(v[0], v[1], v[2], v[3]);
+    } else {
+        for (int k = 0; k < count; ++k) state[s + (uint32_t)k] = v[k];
     }
+}
+
+// Every site's parent becomes its root (for the readers of labels and sizes).
+template <int D, bool SMALL>
+__global__ void __launch_bounds__(kThreads) flatten_kernel(ClusterArgs a) {
+    // (the pass has stored each local root's root at the local root)
+    using T = Tile<D, SMALL>;
+    tile_relabel<T, uint8_t>(
+        a, [](int32_t) { return (uint8_t)0; },
+        [&](uint32_t s, int count, const uint32_t (&r)[4], const uint8_t *, const T &t, uint32_t s_tile) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k < count) a.parent[s + (uint32_t)k] = a.parent[t.site(s_tile, r[k])];
+        });
+}
+
+// keyed (cluster_relabel.wgsl:72-89), every cluster
+template <int D, bool SMALL>
+__global__ void __launch_bounds__(kThreads) relabel_keyed_kernel(ClusterArgs a) {
+    const uint32_t q = (uint32_t)a.q;
+    const bool forced = a.relabel == PLQ_RELABEL_FORCED;
+    using T = Tile<D, SMALL>;
+    tile_relabel<T, uint8_t>(
+        a,
+        [&](int32_t root) {
+            // the forced change's step, or the label itself
+            const float u = __fmul_rn((float)keyed24(a.seed32 ^ kRootSalt, (uint32_t)root, a.sweep32),
+                                      5.9604644775390625e-8f);
+            const uint32_t range = forced ? q - 1u : q;
+            const uint32_t draw = __float2uint_rz(__fmul_rn(u, (float)range));
+            return (uint8_t)(draw >= range ? range - 1u : draw);
+        },
+        [&](uint32_t s, int count, const uint32_t (&r)[4], const uint8_t *value, const T &, uint32_t) {
+            uint8_t v[4] = {value[r[0]], value[r[1]], value[r[2]], value[r[3]]};
+            if (forced)
+                for (int k = 0; k < count; ++k) v[k] = (uint8_t)((a.state[s + (uint32_t)k] + 1u + v[k]) % q);
+            store_row(a.state, s, count, v);
+        });
 }
 
 // rand 0.10 random_range(0..range) for range < 2^32 whose first draw is the
@@ -655,26 +942,22 @@ __global__ void __launch_bounds__(kThreads) root_rank_kernel(ClusterArgs a) {
         return;
     }
     const int64_t s0 = chunk * kChunk + (int64_t)threadIdx.x * kSitesPerThread;
+    // the tiles' local roots are marked in fresh (tile_hook_kernel); those still their own parent are roots
     int count = 0;
     uint32_t mask = 0;
-    if (s0 + kSitesPerThread <= n) {  // s0 is a multiple of 8: two aligned 16-byte loads
-        const int4 lo = *reinterpret_cast<const int4 *>(a.parent + s0);
-        const int4 hi = *reinterpret_cast<const int4 *>(a.parent + s0 + 4);
-        const int32_t par[kSitesPerThread] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    if (s0 + kSitesPerThread <= n) {  // s0 is a multiple of 8
+        const uint64_t f = *reinterpret_cast<const uint64_t *>(a.fresh + s0);
 #pragma unroll
-        for (int i = 0; i < kSitesPerThread; ++i)
-            if (par[i] == (int32_t)(s0 + i)) mask |= 1u << i;
-        count = __popc(mask);
+        for (int i = 0; i < kSitesPerThread; ++i) mask |= (uint32_t)((f >> (8 * i)) & 1u) << i;
     } else {
 #pragma unroll
-        for (int i = 0; i < kSitesPerThread; ++i) {
-            int64_t s = s0 + i;
-            if (s < n && a.parent[s] == (int32_t)s) {
-                mask |= 1u << i;
-                ++count;
-            }
-        }
+        for (int i = 0; i < kSitesPerThread; ++i)
+            if (s0 + i < n) mask |= (uint32_t)(a.fresh[s0 + i] & 1u) << i;
     }
+#pragma unroll
+    for (int i = 0; i < kSitesPerThread; ++i)
+        if (((mask >> i) & 1u) && a.parent[s0 + i] != (int32_t)(s0 + i)) mask &= ~(1u << i);
+    count = __popc(mask);
     int total;
     bool ok;
     uint64_t excl = chunk_scan(a, chunk, count, total, ok);
@@ -710,9 +993,15 @@ __global__ void __launch_bounds__(kThreads) root_rank_kernel(ClusterArgs a) {
 // stream: each root draws its cluster's fresh label (ClusterUpdate::fresh_label,
 // updater.rs:507-521) at bond_end + rank + (known second draws before it),
 // jumping from its root_rank chunk's first label draw.
-__global__ void root_draw_kernel(ClusterArgs a) {
-    const int64_t n = a.g.n_sites;
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
+template <int D, bool SMALL>
+__global__ void __launch_bounds__(kThreads) root_draw_kernel(ClusterArgs a) {
+    using T = Tile<D, SMALL>;
+    const T t(a.g);
+    int xt[3];
+    const uint32_t s_tile = t.origin(blockIdx.x, xt);
+    for (uint32_t li = threadIdx.x; li < T::kSites; li += kThreads) {
+        if (!t.inside(xt, li) || a.local_root[(size_t)blockIdx.x * T::kSites + li] != li) continue;
+        const int64_t s = t.site(s_tile, li);
         if (a.parent[s] != (int32_t)s) continue;
         int32_t r = a.rank[s];
         int before = 0;
@@ -729,19 +1018,15 @@ __global__ void root_draw_kernel(ClusterArgs a) {
     }
 }
 
-__global__ void apply_fresh_kernel(ClusterArgs a) {
-    const int64_t n = a.g.n_sites;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t s0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s0 < n; s0 += stride * kRootBatch) {
-        int32_t roots[kRootBatch];
-        take_roots(a, s0, stride, n, roots);
-        uint8_t f[kRootBatch];
-#pragma unroll
-        for (int k = 0; k < kRootBatch; ++k) f[k] = s0 + k * stride < n ? a.fresh[roots[k]] : 0;
-#pragma unroll
-        for (int k = 0; k < kRootBatch; ++k)
-            if (s0 + k * stride < n) a.state[s0 + k * stride] = f[k];
-    }
+template <int D, bool SMALL>
+__global__ void __launch_bounds__(kThreads) apply_fresh_kernel(ClusterArgs a) {
+    using T = Tile<D, SMALL>;
+    tile_relabel<T, uint8_t>(
+        a, [&](int32_t root) { return a.fresh[root]; },
+        [&](uint32_t s, int count, const uint32_t (&r)[4], const uint8_t *value, const T &, uint32_t) {
+            const uint8_t v[4] = {value[r[0]], value[r[1]], value[r[2]], value[r[3]]};
+            store_row(a.state, s, count, v);
+        });
 }
 
 __global__ void finish_pos_kernel(Control *ctrl, int n_events) {
@@ -832,15 +1117,34 @@ __global__ void __launch_bounds__(kBfsThreads) wolff_bfs_kernel(ClusterArgs a) {
 }
 
 // ------------------------------------------------------------ sizes
-// Cluster sizes: one atomic per distinct root among a warp's 32 sites (a big
-// cluster's root would otherwise take one atomic per site).
-__global__ void sizes_kernel(const int32_t *parent, int32_t *size, int64_t n) {
+// Cluster sizes.  A warp adds up the sites of each distinct root among its 32,
+// into its CTA's table of recent roots where that root has (or finds free) its
+// slot, else in memory; the table is added to memory at the end.  A cluster
+// that holds a good part of the lattice so takes one global atomic per CTA: with
+// one per warp on the same address this kernel took 534 of the 617 us of a
+// histogram of 4096^2 at beta_c (now 240, the flattening of the labels included).
+constexpr int kSizeSlots = 512;
+__global__ void __launch_bounds__(kThreads) sizes_kernel(const int32_t *parent, int32_t *size, int64_t n) {
+    __shared__ int32_t s_root[kSizeSlots], s_count[kSizeSlots];
+    for (int i = threadIdx.x; i < kSizeSlots; i += blockDim.x) {
+        s_root[i] = -1;
+        s_count[i] = 0;
+    }
+    __syncthreads();
     const int64_t n_pad = (n + 31) & ~(int64_t)31;  // whole warps per iteration: the match below is warp-wide
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n_pad; s += (int64_t)gridDim.x * blockDim.x) {
         const int32_t r = s < n ? parent[s] : -1;
         const unsigned peers = __match_any_sync(0xffffffffu, r);
-        if (r >= 0 && (int)(threadIdx.x & 31u) == __ffs(peers) - 1) atomicAdd(&size[r], __popc(peers));
+        if (r >= 0 && (int)(threadIdx.x & 31u) == __ffs(peers) - 1) {
+            const int slot = (int)(((uint32_t)r * 0x9e3779b1u) >> 23);  // kSizeSlots = 2^9
+            const int32_t held = atomicCAS(&s_root[slot], -1, r);
+            if (held == -1 || held == r) atomicAdd(&s_count[slot], __popc(peers));
+            else atomicAdd(&size[r], __popc(peers));
+        }
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kSizeSlots; i += blockDim.x)
+        if (s_count[i]) atomicAdd(&size[s_root[i]], s_count[i]);
 }
 // Clusters per size bin [2^k, 2^(k+1)): counted per CTA in shared memory (bins
 // 0..31 cover every int32 size), one global atomic per bin per CTA.
@@ -864,6 +1168,7 @@ __global__ void size_hist_kernel(const int32_t *parent, const int32_t *size, int
 struct ClusterDev {
     uint8_t *bonds = nullptr;
     int32_t *parent = nullptr;
+    uint16_t *local_root = nullptr;
     uint8_t *fresh = nullptr;
     int32_t *rank = nullptr;
     ClusterArgs::ChunkBase *chunk_base = nullptr;
@@ -871,7 +1176,8 @@ struct ClusterDev {
     int32_t *queue = nullptr;
     unsigned long long *desc = nullptr;
     int64_t n_chunks = 0;
-    int64_t n_tiles = 0;  // CTAs of tile_hook_kernel
+    int64_t n_tiles = 0;  // CTAs of the kernels that take a tile each
+    bool small_tiles = false;
     int32_t *events = nullptr;
     int *first_new = nullptr;
     int32_t *sizes = nullptr;
@@ -880,6 +1186,7 @@ struct ClusterDev {
     uint64_t lookback_launches = 0;
     std::vector<int32_t> host_events;
     bool decomposed = false;
+    bool flat = false;  // every site's parent is its root (flatten_kernel has run since the last sweep)
 };
 
 unsigned grid_stride_blocks(int64_t n) {
@@ -895,6 +1202,7 @@ ClusterArgs cluster_args(plq_chain *c) {
     a.state = c->d_state;
     a.bonds = cd->bonds;
     a.parent = cd->parent;
+    a.local_root = cd->local_root;
     a.fresh = cd->fresh;
     a.rank = cd->rank;
     a.chunk_base = cd->chunk_base;
@@ -928,8 +1236,34 @@ bool label_range_is_power_of_two(const plq_chain *c) {
     return (range & (range - 1u)) == 0u;
 }
 
-template <int D>
-int sweep_d(plq_chain *c, uint64_t sweeps) {
+// The kernels of one tile size (a CTA per tile, and the boundary unions).
+template <int D, bool SMALL>
+struct TileKernels {
+    static void label(const ClusterArgs &a, bool keyed, unsigned tiles, unsigned blocks, cudaStream_t st) {
+        if (keyed) {
+            tile_hook_kernel<D, SMALL, true><<<tiles, kThreads, 0, st>>>(a);
+            boundary_hook_kernel<D, SMALL, true><<<blocks, kThreads, 0, st>>>(a);
+        } else {
+            tile_hook_kernel<D, SMALL, false><<<tiles, kThreads, 0, st>>>(a);
+            boundary_hook_kernel<D, SMALL, false><<<blocks, kThreads, 0, st>>>(a);
+        }
+    }
+    static void relabel_keyed(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
+        relabel_keyed_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
+    }
+    static void root_draw(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
+        root_draw_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
+    }
+    static void apply_fresh(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
+        apply_fresh_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
+    }
+    static void flatten(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
+        flatten_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
+    }
+};
+
+template <int D, class K>
+int sweep_t(plq_chain *c, uint64_t sweeps) {
     ClusterDev *cd = static_cast<ClusterDev *>(c->cl);
     const bool stream = c->desc.rng == PLQ_RNG_STREAM;
     const int64_t n = c->n_sites;
@@ -956,17 +1290,15 @@ int sweep_d(plq_chain *c, uint64_t sweeps) {
             // PCG stream: the bond draws sit at scanned positions, so they are made in one pass
             lookback(a);
             bonds_kernel<D, true><<<(unsigned)cd->n_chunks, kThreads, 0, c->stream>>>(a);
-            tile_hook_kernel<D, false><<<(unsigned)cd->n_tiles, kThreads, 0, c->stream>>>(a);
-            boundary_hook_kernel<D, false><<<gs, kThreads, 0, c->stream>>>(a);
+            K::label(a, false, (unsigned)cd->n_tiles, gs, c->stream);
             c->launches += 3;
         } else {
             // keyed: each bond is a closed form of its index, evaluated where it is used
-            tile_hook_kernel<D, true><<<(unsigned)cd->n_tiles, kThreads, 0, c->stream>>>(a);
-            boundary_hook_kernel<D, true><<<gs, kThreads, 0, c->stream>>>(a);
+            K::label(a, true, (unsigned)cd->n_tiles, gs, c->stream);
             c->launches += 2;
         }
         if (!stream) {
-            relabel_keyed_kernel<<<gs, kThreads, 0, c->stream>>>(a);
+            K::relabel_keyed(a, (unsigned)cd->n_tiles, c->stream);
             c->launches++;
         } else if (label_range_is_power_of_two(c)) {
             // rand's range sampler never takes a second draw for a power-of-two range
@@ -975,7 +1307,7 @@ int sweep_d(plq_chain *c, uint64_t sweeps) {
             // sweep needs no round-trip to the host
             lookback(a);
             root_rank_kernel<D><<<(unsigned)cd->n_chunks, kThreads, 0, c->stream>>>(a);
-            apply_fresh_kernel<<<gs, kThreads, 0, c->stream>>>(a);
+            K::apply_fresh(a, (unsigned)cd->n_tiles, c->stream);
             finish_pos_kernel<<<1, 1, 0, c->stream>>>(c->d_ctrl, 0);
             c->launches += 3;
         } else {
@@ -992,7 +1324,7 @@ int sweep_d(plq_chain *c, uint64_t sweeps) {
                     cudaMemcpyAsync(cd->first_new, &none, sizeof none, cudaMemcpyHostToDevice, c->stream);
                     cudaMemcpyAsync(cd->events, cd->host_events.data(), sizeof(int32_t) * a.n_events,
                                     cudaMemcpyHostToDevice, c->stream);
-                    root_draw_kernel<<<gs, kThreads, 0, c->stream>>>(a);
+                    K::root_draw(a, (unsigned)cd->n_tiles, c->stream);
                     c->launches++;
                 }
                 int first = none;
@@ -1004,7 +1336,7 @@ int sweep_d(plq_chain *c, uint64_t sweeps) {
                     return plq_fail(PLQ_EDEVICE, "too many two-draw label events in one sweep");
                 cd->host_events.insert(std::upper_bound(cd->host_events.begin(), cd->host_events.end(), first), first);
             }
-            apply_fresh_kernel<<<gs, kThreads, 0, c->stream>>>(a);
+            K::apply_fresh(a, (unsigned)cd->n_tiles, c->stream);
             finish_pos_kernel<<<1, 1, 0, c->stream>>>(c->d_ctrl, (int)cd->host_events.size());
             c->launches += 2;
         }
@@ -1012,8 +1344,15 @@ int sweep_d(plq_chain *c, uint64_t sweeps) {
         if (e != cudaSuccess) return plq_fail(PLQ_ECUDA, std::string("cluster sweep: ") + cudaGetErrorString(e));
         c->sweeps_done++;
         cd->decomposed = true;
+        cd->flat = false;
     }
     return PLQ_OK;
+}
+
+template <int D>
+int sweep_d(plq_chain *c, uint64_t sweeps) {
+    return static_cast<ClusterDev *>(c->cl)->small_tiles ? sweep_t<D, TileKernels<D, true>>(c, sweeps)
+                                                        : sweep_t<D, TileKernels<D, D == 1>>(c, sweeps);
 }
 
 }  // namespace
@@ -1049,10 +1388,16 @@ int cluster_create(plq_chain *c) {
     cd->kp53 = lo53;
     c->pass_cap = (c->desc.flags & PLQ_FLAG_TINY_PASS_CAP) ? 1 : std::min<int64_t>(n + 64, 1 << 30);
     cd->n_chunks = (n + kChunk - 1) / kChunk;
-    {
-        auto tile = [](int64_t L) { const int64_t p2 = L & -L; return p2 < kTileMax ? p2 : (int64_t)kTileMax; };
-        const int64_t t0 = tile(c->g.L[0]), t1 = c->d >= 2 ? tile(c->g.L[1]) : 1;
-        cd->n_tiles = n / (t0 * t1);
+    size_t tile_sites = 0;
+    auto tiles = [&](auto large, auto small_t, bool is_large) {
+        cd->small_tiles = !is_large;
+        cd->n_tiles = is_large ? large.tiles(n) : small_t.tiles(n);
+        tile_sites = (size_t)cd->n_tiles * (is_large ? decltype(large)::kSites : decltype(small_t)::kSites);
+    };
+    switch (c->d) {  // (d > 3 has the tiles of d = 3)
+        case 1: tiles(Tile<1, false>(c->g), Tile<1, true>(c->g), false); break;
+        case 2: tiles(Tile<2, false>(c->g), Tile<2, true>(c->g), large_tiles<2>(c->g, c->ctx->sm_count)); break;
+        default: tiles(Tile<3, false>(c->g), Tile<3, true>(c->g), large_tiles<3>(c->g, c->ctx->sm_count)); break;
     }
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void **p, size_t bytes) {
@@ -1065,6 +1410,7 @@ int cluster_create(plq_chain *c) {
     } else {
         alloc((void **)&cd->bonds, (size_t)n);
         alloc((void **)&cd->parent, sizeof(int32_t) * (size_t)n);
+        alloc((void **)&cd->local_root, sizeof(uint16_t) * tile_sites);
         alloc((void **)&cd->desc, sizeof(unsigned long long) * (size_t)cd->n_chunks);
         if (e == cudaSuccess)
             e = cudaMemsetAsync(cd->desc, 0, sizeof(unsigned long long) * (size_t)cd->n_chunks, c->stream);
@@ -1101,7 +1447,7 @@ int cluster_sweep(plq_chain *c) { return cluster_sweep_n(c, 1); }
 void cluster_free(plq_chain *c) {
     ClusterDev *cd = static_cast<ClusterDev *>(c->cl);
     if (!cd) return;
-    void *ptrs[] = {cd->bonds, cd->parent, cd->fresh, cd->rank, cd->chunk_base, cd->stamp, cd->queue,
+    void *ptrs[] = {cd->bonds, cd->parent, cd->local_root, cd->fresh, cd->rank, cd->chunk_base, cd->stamp, cd->queue,
                     cd->desc, cd->events, cd->first_new, cd->sizes};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -1109,9 +1455,34 @@ void cluster_free(plq_chain *c) {
     c->cl = nullptr;
 }
 
+template <int D>
+static void flatten_d(plq_chain *c) {
+    ClusterDev *cd = static_cast<ClusterDev *>(c->cl);
+    if (cd->small_tiles) TileKernels<D, true>::flatten(cluster_args(c), (unsigned)cd->n_tiles, c->stream);
+    else TileKernels<D, D == 1>::flatten(cluster_args(c), (unsigned)cd->n_tiles, c->stream);
+}
+
+static void flatten(plq_chain *c) {
+    ClusterDev *cd = static_cast<ClusterDev *>(c->cl);
+    if (cd->flat) return;
+    switch (c->d) {
+        case 1: flatten_d<1>(c); break;
+        case 2: flatten_d<2>(c); break;
+        case 3: flatten_d<3>(c); break;
+        case 4: flatten_d<4>(c); break;
+        case 5: flatten_d<5>(c); break;
+        case 6: flatten_d<6>(c); break;
+        case 7: flatten_d<7>(c); break;
+        default: flatten_d<8>(c); break;
+    }
+    c->launches++;
+    cd->flat = true;
+}
+
 int cluster_labels(plq_chain *c, int32_t *out) {
     ClusterDev *cd = static_cast<ClusterDev *>(c->cl);
     if (!cd || !cd->decomposed) return plq_fail(PLQ_EINVAL, "no decomposition yet (run a Swendsen-Wang sweep first)");
+    flatten(c);
     cudaError_t e = cudaMemcpyAsync(out, cd->parent, sizeof(int32_t) * (size_t)c->n_sites, cudaMemcpyDeviceToHost,
                                     c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -1142,6 +1513,7 @@ int cluster_size_histogram(plq_chain *c, int64_t *hist, int32_t nbins) {
         if (e != cudaSuccess) return plq_fail(PLQ_ENOMEM, cudaGetErrorString(e));
         cudaMemsetAsync(cd->sizes, 0, sizeof(int32_t) * (size_t)n, c->stream);
         cudaMemsetAsync(dh, 0, sizeof(long long) * (size_t)nbins, c->stream);
+        flatten(c);
         sizes_kernel<<<grid_stride_blocks(n), kThreads, 0, c->stream>>>(cd->parent, cd->sizes, n);
         size_hist_kernel<<<grid_stride_blocks(n), kThreads, 0, c->stream>>>(cd->parent, cd->sizes, n, dh, nbins);
         c->launches += 2;
