@@ -31,11 +31,10 @@
 //               loop.
 //
 // Wolff on the keyed stream: the reference relabels the cluster of a keyed
-// seed site in the full decomposition (cluster_relabel.wgsl:55-66).  Here a
-// frontier BFS from the seed site over lazily evaluated keyed bonds finds the
-// same component (work proportional to the cluster), its minimum site is the
-// root the forced change is keyed on.  One CTA runs all requested updates in
-// one launch.  Wolff on the PCG stream (draws in grow_cluster's FIFO order)
+// seed site in the full decomposition (cluster_relabel.wgsl:55-66).  Here one
+// persistent launch runs all requested updates: a CTA grows the cluster from
+// the seed site for a few generations while the others label the tiles
+// (wolff_kernel); its minimum site is the root the forced change is keyed on.  Wolff on the PCG stream (draws in grow_cluster's FIFO order)
 // is sequential by definition and is not run on the device.
 //
 // Every loop that waits or retries has an iteration cap; hitting one sets a
@@ -62,7 +61,6 @@ constexpr int kSitesPerThread = 8;
 constexpr int kChunk = kThreads * kSitesPerThread;
 constexpr int kSpinLimit = 1 << 22;
 constexpr int kMaxEvents = 64;
-constexpr int kBfsThreads = 1024;
 constexpr unsigned long long kDescAgg = 1ull, kDescPrefix = 2ull;
 
 struct ClusterArgs {
@@ -76,8 +74,6 @@ struct ClusterArgs {
         u128 st;           // the chunk's first root (no second draws before it) and that root's rank
         int64_t rank0, pad;
     } *chunk_base;
-    uint32_t *stamp;
-    int32_t *queue;
     Geom g;
     int q;
     int extent, relabel;
@@ -305,15 +301,6 @@ __global__ void __launch_bounds__(kThreads) bonds_kernel(ClusterArgs a) {
     if (row8 && s0 < n) *reinterpret_cast<uint64_t *>(a.bonds + s0) = opened;
 }
 
-// The keyed bond (s, mu) to the +mu neighbour `nb`, evaluated where it is
-// used (no bond array on the keyed stream): open iff the two sites agree and
-// the bond's keyed draw is below p (cluster_prelude.wgsl:61-80).
-template <int D>
-__device__ __forceinline__ bool keyed_bond(const ClusterArgs &a, int64_t s, int mu, int64_t nb) {
-    return a.state[s] == a.state[nb] &&
-           keyed24(a.seed32 ^ kBondKey, (uint32_t)(s * D + mu), a.sweep32) < a.kp24;
-}
-
 // ------------------------------------------------------------ 2. labels
 __device__ __forceinline__ int32_t find_root(int32_t *parent, int32_t x, int cap, Control *ctrl) {
     int32_t p = ld_relaxed32(&parent[x]);
@@ -392,6 +379,7 @@ struct Tile {  // block (per warp): 32 x BY x BZ; tile: WX x WY x WZ blocks
                          WZ = D >= 3 ? 2 : 1;
     static constexpr int TX = 32 * WX, TY = BY * WY, TZ = BZ * WZ;
     static constexpr int kSites = TX * TY * TZ;
+    static constexpr int kDims = D;
     static constexpr int G = D == 2 ? 8 : BY;  // rows whose bonds are made together
     static_assert(WX * WY * WZ * 32 == kThreads, "a warp per block");
     static_assert(kSites <= 65536 && (BY * BZ) % G == 0 && BY * BZ <= 32, "16-bit local roots, 32 rows a block");
@@ -453,8 +441,8 @@ bool large_tiles(const Geom &g, int sm_count) {
 // (kp24 = 0, no bond opens, has no T: some() says so, once for a group of draws.)
 struct BondCut {
     uint32_t seed, mix, T, X;
-    __device__ __forceinline__ explicit BondCut(const ClusterArgs &a)
-        : seed(a.seed32 ^ kBondKey), mix(keyed_mix(a.sweep32)), T((a.kp24 << 8) - 1u),
+    __device__ __forceinline__ BondCut(const ClusterArgs &a, uint32_t sweep)
+        : seed(a.seed32 ^ kBondKey), mix(keyed_mix(sweep)), T((a.kp24 << 8) - 1u),
           X(((a.kp24 << 8) - 1u) >> 16) {}
     __device__ __forceinline__ bool open(uint32_t bond) const {
         return (lowbias32_open(lowbias32_head(seed ^ bond) ^ mix) ^ X) <= T;
@@ -508,17 +496,25 @@ __device__ __forceinline__ void edge_unite(int32_t *p, bool open, int32_t u, int
     if (open && !repeat && pu != pv) lunite(p, pu, pv, cap, ctrl);
 }
 
+template <class T>
+struct LabelShared {
+    static constexpr int kBlock = 32 * T::BY * T::BZ;
+    static constexpr int kFurther = T::kDims >= 3 ? 2 * kBlock : T::kDims == 2 ? kBlock : 1;
+    int32_t p[T::kSites];
+    uint16_t further[kThreads / 32][kFurther];
+};
+
+// Labels tile `tile`; the CTA may reuse `sm` at once.
 template <int D, bool SMALL, bool KEYED>
-__global__ void __launch_bounds__(kThreads, D == 2 && !SMALL ? 5 : 1) tile_hook_kernel(ClusterArgs a) {
+__device__ __forceinline__ void label_tile(const ClusterArgs &a, uint32_t sweep, uint32_t tile,
+                                           LabelShared<Tile<D, SMALL>> &sm) {
     using T = Tile<D, SMALL>;
     constexpr int BY = T::BY, BZ = T::BZ, TX = T::TX, TY = T::TY, TZ = T::TZ, G = T::G;
-    constexpr int kBlock = 32 * BY * BZ, kFurther = D >= 3 ? 2 * kBlock : D == 2 ? kBlock : 1;
-    __shared__ int32_t p[T::kSites];
-    __shared__ uint16_t s_further[kThreads / 32][kFurther];
+    int32_t *p = sm.p;
     const T t(a.g);
     const int L0 = t.L[0], L1 = t.L[1], L2 = t.L[2];
     int xt[3];
-    const uint32_t s_tile = t.origin(blockIdx.x, xt);
+    const uint32_t s_tile = t.origin(tile, xt);
     const int cap = a.cap < T::kSites + 64 ? a.cap : T::kSites + 64;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int wx = wid % T::WX, wy = (wid / T::WX) % T::WY, wz = wid / (T::WX * T::WY);
@@ -529,7 +525,7 @@ __global__ void __launch_bounds__(kThreads, D == 2 && !SMALL ? 5 : 1) tile_hook_
     const uint32_t s00 = s_tile + (uint32_t)lz0 * plane + (uint32_t)(ly0 * L0 + lx);
     const int li00 = (lz0 * TY + ly0) * TX + lx;
     const uint32_t le = 0xffffffffu >> (31 - lane);
-    const BondCut cut(a);
+    const BondCut cut(a, sweep);
     const bool x_in_tile = x + 1 < L0 && lx + 1 < TX;  // the +x neighbour is in the tile
 
     // ---- the block's rows in order: labels from the row before and the plane before
@@ -537,7 +533,7 @@ __global__ void __launch_bounds__(kThreads, D == 2 && !SMALL ? 5 : 1) tile_hook_
     // block: about one site in ten has one, and a list keeps whole warps busy uniting them
     constexpr uint32_t kToPlane = 0x8000u;
     static_assert(D < 3 || T::kSites <= 0x8000, "a bit beside the place");
-    uint16_t *further = s_further[wid];
+    uint16_t *further = sm.further[wid];
     int n_further = 0;
     uint32_t mine = 0;  // rows whose label is this lane's own site
     auto list = [&](bool mine, uint32_t entry) {
@@ -686,8 +682,7 @@ __global__ void __launch_bounds__(kThreads, D == 2 && !SMALL ? 5 : 1) tile_hook_
         if (r != li) p[li] = r;
     }
     __syncthreads();
-    if (!in_x) return;
-    uint16_t *roots = a.local_root + (size_t)blockIdx.x * T::kSites;
+    uint16_t *roots = a.local_root + (size_t)tile * T::kSites;
 #pragma unroll 1
     for (int jz = 0; jz < BZ; ++jz) {
         if (D >= 3 && z0 + jz >= L2) break;
@@ -697,11 +692,19 @@ __global__ void __launch_bounds__(kThreads, D == 2 && !SMALL ? 5 : 1) tile_hook_
             const int li = li00 + (jz * TY + jy) * TX;
             const int32_t r = p[p[li]];
             const uint32_t s = s00 + (uint32_t)jz * plane + (uint32_t)(jy * L0);
-            roots[li] = (uint16_t)r;
-            if (r == li) a.parent[s] = (int32_t)s;
-            if (!KEYED) a.fresh[s] = r == li ? 1 : 0;  // root_rank_kernel's candidates, in site order
+            if (in_x) {
+                roots[li] = (uint16_t)r;
+                if (r == li) a.parent[s] = (int32_t)s;
+                if (!KEYED) a.fresh[s] = r == li ? 1 : 0;  // root_rank_kernel's candidates, in site order
+            }
         }
     }
+}
+
+template <int D, bool SMALL, bool KEYED>
+__global__ void __launch_bounds__(kThreads, D == 2 && !SMALL ? 5 : 1) tile_hook_kernel(ClusterArgs a) {
+    __shared__ LabelShared<Tile<D, SMALL>> sm;
+    label_tile<D, SMALL, KEYED>(a, a.sweep32, blockIdx.x, sm);
 }
 
 // Global unions for the open bonds that leave their tile: of the tiles' last
@@ -710,9 +713,10 @@ __global__ void __launch_bounds__(kThreads, D == 2 && !SMALL ? 5 : 1) tile_hook_
 // whose ends' local roots are the lane before's leaves the union to that lane:
 // along a tile edge a large cluster meets another at many sites.
 template <int D, bool SMALL, bool KEYED>
-__global__ void __launch_bounds__(kThreads) boundary_hook_kernel(ClusterArgs a) {
+__device__ __forceinline__ void unite_edges(const ClusterArgs &a, uint32_t sweep) {
     using T = Tile<D, SMALL>;
     const T t(a.g);
+    const BondCut cut(a, sweep);
     const int64_t n = a.g.n_sites;
     const uint32_t L0 = (uint32_t)t.L[0], L1 = (uint32_t)t.L[1], L2 = (uint32_t)t.L[2];
     const uint32_t rows = (uint32_t)(n / L0), planes = rows / L1;  // planes: over every direction past 1
@@ -754,7 +758,10 @@ __global__ void __launch_bounds__(kThreads) boundary_hook_kernel(ClusterArgs a) 
 #pragma unroll
             for (int m = 0; m < D; ++m)
                 if (m == mu) nb = nbr_plus(a.g, s, x, m);
-            if (KEYED) open = keyed_bond<D>(a, s, mu, nb);
+            // keyed: open iff the two sites agree and the bond's draw is below p
+            // (cluster_prelude.wgsl:61-80)
+            if (KEYED)
+                open = a.state[s] == a.state[nb] && BondCut::some(a) && cut.open((uint32_t)(s * D + mu));
             if (open) {
                 pa = (int32_t)t.local_root(a.local_root, (uint32_t)s, x);
 #pragma unroll
@@ -767,6 +774,11 @@ __global__ void __launch_bounds__(kThreads) boundary_hook_kernel(ClusterArgs a) 
         const bool repeat = lane > 0 && qa == pa && qb == pb;
         if (open && !repeat && pa != pb) unite(a.parent, pa, pb, a.cap, a.ctrl);
     }
+}
+
+template <int D, bool SMALL, bool KEYED>
+__global__ void __launch_bounds__(kThreads) boundary_hook_kernel(ClusterArgs a) {
+    unite_edges<D, SMALL, KEYED>(a, a.sweep32);
 }
 
 // Read-only find for the passes after the unions: a compressing find could
@@ -790,18 +802,25 @@ __device__ __forceinline__ int32_t find_root_ro(const int32_t *parent, int32_t x
 // walks through it end there), and of_root(root) gives the value of its sites;
 // then out takes the sites of each row four at a time.  Bound by the latency of the
 // walks, hence the list: full warps of walks instead of one lane in eight.
-template <class T, class V, class F, class O>
-__device__ __forceinline__ void tile_relabel(const ClusterArgs &a, F of_root, O out) {
-    __shared__ __align__(16) uint16_t s_root[T::kSites];
-    __shared__ uint16_t s_list[T::kSites];
-    __shared__ V s_value[T::kSites];
-    __shared__ int s_n;
+template <class T>
+struct RelabelShared {
+    alignas(16) uint16_t root[T::kSites];
+    uint16_t list[T::kSites];
+    uint8_t value[T::kSites];
+    int n;
+};
+
+template <class T, class F, class O>
+__device__ __forceinline__ void tile_relabel(const ClusterArgs &a, uint32_t tile, RelabelShared<T> &sm, F of_root, O out) {
+    uint16_t *s_root = sm.root, *s_list = sm.list;
+    uint8_t *s_value = sm.value;
+    int &s_n = sm.n;
     const T t(a.g);
     int xt[3];
-    const uint32_t s_tile = t.origin(blockIdx.x, xt);
+    const uint32_t s_tile = t.origin(tile, xt);
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
-    const uint4 *src = reinterpret_cast<const uint4 *>(a.local_root + (size_t)blockIdx.x * T::kSites);
+    const uint4 *src = reinterpret_cast<const uint4 *>(a.local_root + (size_t)tile * T::kSites);
 #pragma unroll(T::kSites / 8 / kThreads > 4 ? 4 : 1)
     for (uint32_t i = threadIdx.x; i < T::kSites / 8; i += kThreads) {
         const uint4 v = src[i];
@@ -870,8 +889,9 @@ template <int D, bool SMALL>
 __global__ void __launch_bounds__(kThreads) flatten_kernel(ClusterArgs a) {
     // (the pass has stored each local root's root at the local root)
     using T = Tile<D, SMALL>;
-    tile_relabel<T, uint8_t>(
-        a, [](int32_t) { return (uint8_t)0; },
+    __shared__ RelabelShared<T> sm;
+    tile_relabel<T>(
+        a, blockIdx.x, sm, [](int32_t) { return (uint8_t)0; },
         [&](uint32_t s, int count, const uint32_t (&r)[4], const uint8_t *, const T &t, uint32_t s_tile) {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
@@ -885,8 +905,9 @@ __global__ void __launch_bounds__(kThreads) relabel_keyed_kernel(ClusterArgs a) 
     const uint32_t q = (uint32_t)a.q;
     const bool forced = a.relabel == PLQ_RELABEL_FORCED;
     using T = Tile<D, SMALL>;
-    tile_relabel<T, uint8_t>(
-        a,
+    __shared__ RelabelShared<T> sm;
+    tile_relabel<T>(
+        a, blockIdx.x, sm,
         [&](int32_t root) {
             // the forced change's step, or the label itself
             const float u = __fmul_rn((float)keyed24(a.seed32 ^ kRootSalt, (uint32_t)root, a.sweep32),
@@ -1021,8 +1042,9 @@ __global__ void __launch_bounds__(kThreads) root_draw_kernel(ClusterArgs a) {
 template <int D, bool SMALL>
 __global__ void __launch_bounds__(kThreads) apply_fresh_kernel(ClusterArgs a) {
     using T = Tile<D, SMALL>;
-    tile_relabel<T, uint8_t>(
-        a, [&](int32_t root) { return a.fresh[root]; },
+    __shared__ RelabelShared<T> sm;
+    tile_relabel<T>(
+        a, blockIdx.x, sm, [&](int32_t root) { return a.fresh[root]; },
         [&](uint32_t s, int count, const uint32_t (&r)[4], const uint8_t *value, const T &, uint32_t) {
             const uint8_t v[4] = {value[r[0]], value[r[1]], value[r[2]], value[r[3]]};
             store_row(a.state, s, count, v);
@@ -1033,87 +1055,271 @@ __global__ void finish_pos_kernel(Control *ctrl, int n_events) {
     ctrl->pos[0] = ctrl->pos[1] + ctrl->scratch[0] + (unsigned long long)n_events;
 }
 
-// ------------------------------------------------------- Wolff (keyed BFS)
-template <int D>
-__global__ void __launch_bounds__(kBfsThreads) wolff_bfs_kernel(ClusterArgs a) {
-    __shared__ int s_tail, s_min;
-    __shared__ int s_lvl_begin, s_lvl_end;
-    const int64_t n = a.g.n_sites;
+// ------------------------------------------------------- Wolff (keyed)
+// An update by growth from the seed site is a chain of generations, some 70 for
+// a critical 3D cluster of 10^4 sites and over 1000 for a 2D one of 10^5: at
+// about a microsecond each, growth takes many times what labelling the whole
+// lattice does on all SMs (2D Ising 1024^2: 3.9 ms an update against 0.034).
+// But far from criticality, and for many seeds at it, the cluster is a few
+// sites, which a few generations find.  So one CTA of a persistent launch grows
+// each update's cluster and goes on to the next as long as they are small; at
+// generation kAnnounce it calls the others, which label the tiles as in a
+// Swendsen-Wang sweep while it grows on to kGrowGenerations (they stop when the
+// growth has ended first).  A cluster that outgrew the limits is the one the
+// seed site has in the decomposition.  Grid barriers: none for an update of
+// fewer generations, one where the growth ended after the call, three for a
+// large cluster.
+//
+// us per update, growth on one CTA / this, in equilibrium at beta_c: 3D Ising
+// 128^3 536 / 45, 48 x 50 x 54 226 / 21, 2D Ising 1024^2 3750 / 35, 194 x 172
+// 592 / 26, 32 x 26 87 / 23, 3D Potts q = 3 80^3 60 / 19; 3D Ising 128^3 at
+// beta = 0.1 4.1 / 3.0.  Calling at generation 4 was 2 us faster on the smallest
+// lattices and 1.5 us slower on the hot one.
+constexpr int kAnnounce = 6;
+constexpr int kGrowGenerations = 12;
+constexpr uint32_t kGrowMembers = 1024;
+constexpr uint32_t kGrowTable = 4096;  // members' hash table: never more than half full
+static_assert(kGrowMembers + kThreads <= kGrowTable / 2, "room for a pass past the limit");
+
+struct GrowShared {
+    int32_t table[kGrowTable];
+    int32_t queue[kGrowMembers];
+    uint32_t tail, min_site;
+};
+
+// Device-side state of a Wolff chain's launches.
+struct WolffSync {
+    unsigned int count, gen;      // the grid barrier's arrivals and generation
+    unsigned long long call;      // the update the CTAs are called to label (increasing over all launches)
+    unsigned long long small[2];  // by update parity: the called update whose cluster the growth found whole
+};
+
+// Grid barrier (all CTAs are co-resident: a cooperative launch); bounded.
+__device__ void wolff_barrier(WolffSync *w, Control *ctrl) {
+    __syncthreads();
+    if (threadIdx.x == 0 && gridDim.x > 1) {
+        volatile unsigned int *gen = &w->gen;
+        const unsigned int g = *gen;
+        __threadfence();
+        if (atomicAdd(&w->count, 1u) == gridDim.x - 1) {
+            atomicExch(&w->count, 0u);
+            __threadfence();
+            atomicAdd(&w->gen, 1u);
+        } else {
+            for (int spins = 0; *gen == g;) {
+                if (++spins > (1 << 24)) {
+                    atomicOr(&ctrl->status, kStatusLookbackTimeout);
+                    break;
+                }
+                __nanosleep(20);
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+}
+
+// The new state of the cluster rooted at `root` (cluster_relabel.wgsl:72-89).
+__device__ __forceinline__ uint8_t wolff_next(const ClusterArgs &a, uint32_t sweep, uint32_t root, uint32_t cur) {
     const uint32_t q = (uint32_t)a.q;
-    for (uint64_t up = 0; up < a.updates; ++up) {
-        const uint32_t sweep = a.sweep32 + (uint32_t)up;
-        const uint32_t epoch = sweep + 1u;
-        // seed site (cluster_relabel.wgsl:55-61)
-        float us = __fmul_rn((float)keyed24(a.seed32 ^ kSeedSalt, 0u, sweep), 5.9604644775390625e-8f);
-        uint32_t seed_site = __float2uint_rz(__fmul_rn(us, (float)(uint32_t)n));
-        if (seed_site >= (uint32_t)n) seed_site = (uint32_t)n - 1u;
-        if (threadIdx.x == 0) {
-            a.queue[0] = (int32_t)seed_site;
-            a.stamp[seed_site] = epoch;
-            s_tail = 1;
-            s_min = (int32_t)seed_site;
-            s_lvl_begin = 0;
-            s_lvl_end = 1;
+    const float u = __fmul_rn((float)keyed24(a.seed32 ^ kRootSalt, root, sweep), 5.9604644775390625e-8f);
+    if (a.relabel == PLQ_RELABEL_FORCED) {
+        uint32_t step = __float2uint_rz(__fmul_rn(u, (float)(q - 1u)));
+        if (step >= q - 1u) step = q - 2u;
+        return (uint8_t)((cur + 1u + step) % q);
+    }
+    uint32_t draw = __float2uint_rz(__fmul_rn(u, (float)q));
+    if (draw >= q) draw = q - 1u;
+    return (uint8_t)draw;
+}
+
+// Calls the waiting CTAs to update `id`: everything this CTA has written is visible to them.
+__device__ __forceinline__ void wolff_call(WolffSync *w, unsigned long long id) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        *(volatile unsigned long long *)&w->call = id;
+    }
+}
+
+// Growth from `seed` within the limits, one thread per (member, direction): true
+// if the whole cluster was found, its members then in sm.queue.  `called`: the
+// other CTAs were called to this update.
+template <int D>
+__device__ bool wolff_grow(const ClusterArgs &a, uint32_t sweep, uint32_t seed, uint8_t cur, GrowShared &sm, WolffSync *w,
+                           unsigned long long id, bool &called) {
+    const BondCut cut(a, sweep);
+    const bool bonds = BondCut::some(a);
+    auto slot_of = [](uint32_t v) { return (v * 0x9e3779b1u) >> 20; };  // kGrowTable = 2^12
+    for (uint32_t i = threadIdx.x; i < kGrowTable; i += kThreads) sm.table[i] = -1;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        sm.table[slot_of(seed)] = (int32_t)seed;
+        sm.queue[0] = (int32_t)seed;
+        sm.tail = 1;
+        sm.min_site = seed;
+    }
+    __syncthreads();
+    uint32_t begin = 0, end = 1;
+    called = false;
+    for (int gen = 0; begin < end && gen < kGrowGenerations && end <= kGrowMembers; ++gen) {
+        if (gen == kAnnounce) {
+            wolff_call(w, id);
+            called = true;
+        }
+        const uint32_t work = (end - begin) * (2u * D);
+        for (uint32_t i = threadIdx.x; i < work; i += kThreads) {
+            const uint32_t k = i % (2u * D), u = (uint32_t)sm.queue[begin + i / (2u * D)];
+            int32_t x[D];
+            site_coords<D>(a.g, u, x);
+            const bool plus = (k & 1u) == 0;
+            uint32_t v = 0;
+#pragma unroll
+            for (int mu = 0; mu < D; ++mu)
+                if ((k >> 1) == (uint32_t)mu) v = (uint32_t)(plus ? nbr_plus(a.g, u, x, mu) : nbr_minus(a.g, u, x, mu));
+            const uint8_t sv = a.state[v];
+            if ((sv == cur) & bonds & cut.open((plus ? u : v) * (uint32_t)D + (k >> 1))) {
+                // (past the limit the growth has failed: the tail only has to stay above it)
+                if (*(volatile uint32_t *)&sm.tail > kGrowMembers) break;
+                uint32_t slot = slot_of(v);
+                int32_t held;
+                while ((held = atomicCAS(&sm.table[slot], -1, (int32_t)v)) != -1 && held != (int32_t)v)
+                    slot = (slot + 1u) % kGrowTable;
+                if (held == -1) {
+                    const uint32_t p = atomicAdd(&sm.tail, 1u);
+                    if (p < kGrowMembers) sm.queue[p] = (int32_t)v;
+                    if (v < sm.min_site) atomicMin(&sm.min_site, v);
+                }
+            }
         }
         __syncthreads();
-        const uint8_t cur = a.state[seed_site];
-        while (true) {
-            int begin = s_lvl_begin, end = s_lvl_end;
-            if (begin >= end) break;
-            for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
-                int64_t u = a.queue[i];
-                int32_t x[D];
-                site_coords<D>(a.g, u, x);
-                // the 2D neighbours' loads, then their stamp exchanges, each issued together so
-                // their latencies overlap; the cluster (a set) does not depend on the order
-                int64_t v[2 * D];
-                uint8_t sv[2 * D];
-#pragma unroll
-                for (int k = 0; k < 2 * D; ++k) {
-                    v[k] = (k & 1) == 0 ? nbr_plus(a.g, u, x, k >> 1) : nbr_minus(a.g, u, x, k >> 1);
-                    sv[k] = a.state[v[k]];
-                }
-                bool join[2 * D];
-#pragma unroll
-                for (int k = 0; k < 2 * D; ++k) {
-                    const uint32_t bond = (uint32_t)(((k & 1) == 0 ? u : v[k]) * D + (k >> 1));
-                    join[k] = sv[k] == cur && keyed24(a.seed32 ^ kBondKey, bond, sweep) < a.kp24;
-                }
-#pragma unroll
-                for (int k = 0; k < 2 * D; ++k)
-                    if (join[k]) join[k] = atomicExch(&a.stamp[v[k]], epoch) != epoch;  // not yet a member
-#pragma unroll
-                for (int k = 0; k < 2 * D; ++k) {
-                    if (!join[k]) continue;
-                    int slot = atomicAdd(&s_tail, 1);
-                    a.queue[slot] = (int32_t)v[k];
-                    atomicMin(&s_min, (int32_t)v[k]);
-                }
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                s_lvl_begin = end;
-                s_lvl_end = s_tail;
-            }
-            __syncthreads();
-        }
-        const int members = s_tail;
-        const uint32_t root = (uint32_t)s_min;
-        float u = __fmul_rn((float)keyed24(a.seed32 ^ kRootSalt, root, sweep), 5.9604644775390625e-8f);
-        uint8_t next;
-        if (a.relabel == PLQ_RELABEL_FORCED) {
-            uint32_t step = __float2uint_rz(__fmul_rn(u, (float)(q - 1u)));
-            if (step >= q - 1u) step = q - 2u;
-            next = (uint8_t)((cur + 1u + step) % q);
-        } else {
-            uint32_t draw = __float2uint_rz(__fmul_rn(u, (float)q));
-            if (draw >= q) draw = q - 1u;
-            next = (uint8_t)draw;
-        }
-        for (int i = threadIdx.x; i < members; i += blockDim.x) a.state[a.queue[i]] = next;
-        if (threadIdx.x == 0) a.ctrl->scratch[1] = (unsigned long long)members;
+        begin = end;
+        end = sm.tail;
         __syncthreads();
     }
+    if (begin < end && !called) {
+        wolff_call(w, id);
+        called = true;
+    }
+    return begin == end;
+}
+
+template <int D, bool SMALL>
+__global__ void __launch_bounds__(kThreads, 4)
+wolff_kernel(ClusterArgs a, WolffSync *w, uint32_t n_tiles, unsigned long long launch) {
+    using T = Tile<D, SMALL>;
+    constexpr size_t kBytes = sizeof(LabelShared<T>) > sizeof(RelabelShared<T>)
+                                  ? (sizeof(LabelShared<T>) > sizeof(GrowShared) ? sizeof(LabelShared<T>) : sizeof(GrowShared))
+                                  : (sizeof(RelabelShared<T>) > sizeof(GrowShared) ? sizeof(RelabelShared<T>) : sizeof(GrowShared));
+    __shared__ __align__(16) unsigned char s_buf[kBytes];
+    __shared__ int s_stop;
+    __shared__ unsigned long long s_call;
+    __shared__ uint32_t s_root, s_flipped;
+    const uint32_t n = (uint32_t)a.g.n_sites;
+    const bool grower = blockIdx.x == 0;  // (there are others: a grid has a CTA per tile and one more, or fills the chip)
+    const unsigned long long base = launch << 32, last = base | 0xFFFFFFFFull;  // (a launch has less than 2^32 - 1 updates)
+    unsigned long long id = base;  // update up is base + up + 1
+    // a CTA that waits for a call reads the word until the growing CTA has been through every
+    // update before it, at a few microseconds each; the limit is some 100 times that
+    const unsigned long long spin_limit = (1ull << 24) + (a.updates << 14);
+    for (;;) {
+        if (grower) {
+            if (id == base + a.updates) break;
+            ++id;
+        } else {
+            if (threadIdx.x == 0) {
+                volatile unsigned long long *call = &w->call;
+                unsigned long long next, spins = 0;
+                while ((next = *call) <= id) {
+                    if (++spins > spin_limit) {
+                        atomicOr(&a.ctrl->status, kStatusLookbackTimeout);
+                        next = last;
+                        break;
+                    }
+                    __nanosleep(50);
+                }
+                __threadfence();
+                s_call = next;
+            }
+            __syncthreads();
+            id = s_call;
+            __syncthreads();
+            if (id == last) break;
+        }
+        const uint32_t sweep = a.sweep32 + (uint32_t)(id - base - 1ull);
+        volatile unsigned long long *small = &w->small[id & 1ull];
+        // seed site (cluster_relabel.wgsl:55-61)
+        const float us = __fmul_rn((float)keyed24(a.seed32 ^ kSeedSalt, 0u, sweep), 5.9604644775390625e-8f);
+        uint32_t seed = __float2uint_rz(__fmul_rn(us, (float)n));
+        if (seed >= n) seed = n - 1u;
+        // (another CTA may read a state the growth has changed already, but then has no use for it)
+        const uint8_t cur = a.state[seed];
+        __syncthreads();
+        if (grower) {
+            GrowShared &sm = *reinterpret_cast<GrowShared *>(s_buf);
+            if (threadIdx.x == 0) a.ctrl->scratch[1] = 0;
+            bool called;
+            const bool whole = wolff_grow<D>(a, sweep, seed, cur, sm, w, id, called);
+            if (whole) {
+                // (the others may be reading states for tiles that no one will use)
+                const uint8_t next = wolff_next(a, sweep, sm.min_site, cur);
+                for (uint32_t i = threadIdx.x; i < sm.tail; i += kThreads) a.state[sm.queue[i]] = next;
+                if (threadIdx.x == 0) {
+                    a.ctrl->scratch[1] = sm.tail;
+                    if (called) *small = id;
+                }
+                __syncthreads();
+                if (!called) continue;
+            }
+        } else {
+            LabelShared<T> &sm = *reinterpret_cast<LabelShared<T> *>(s_buf);
+            for (uint32_t tile = blockIdx.x - 1u; tile < n_tiles; tile += gridDim.x - 1u) {
+                if (threadIdx.x == 0) s_stop = *small == id;
+                __syncthreads();
+                if (s_stop) break;
+                label_tile<D, SMALL, true>(a, sweep, tile, sm);
+                __syncthreads();
+            }
+        }
+        wolff_barrier(w, a.ctrl);
+        if (threadIdx.x == 0) s_stop = *small == id;
+        __syncthreads();
+        if (s_stop) continue;
+        unite_edges<D, SMALL, true>(a, sweep);
+        wolff_barrier(w, a.ctrl);
+        // the seed's cluster takes its new state
+        if (threadIdx.x == 0) {
+            int32_t x[D];
+            site_coords<D>(a.g, seed, x);
+            const T t(a.g);
+            s_root = (uint32_t)find_root_ro(a.parent, (int32_t)t.local_root(a.local_root, seed, x), a.cap, a.ctrl);
+            s_flipped = 0;
+        }
+        __syncthreads();
+        const int32_t root = (int32_t)s_root;
+        const uint8_t next = wolff_next(a, sweep, s_root, cur);
+        uint32_t flipped = 0;
+        RelabelShared<T> &sm = *reinterpret_cast<RelabelShared<T> *>(s_buf);
+        for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+            tile_relabel<T>(
+                a, tile, sm, [&](int32_t r) { return (uint8_t)(r == root ? 1 : 0); },
+                [&](uint32_t s, int count, const uint32_t (&r)[4], const uint8_t *value, const T &, uint32_t) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (k < count && value[r[k]]) {
+                            a.state[s + (uint32_t)k] = next;
+                            ++flipped;
+                        }
+                });
+            __syncthreads();
+        }
+        flipped = __reduce_add_sync(0xffffffffu, flipped);
+        if ((threadIdx.x & 31u) == 0 && flipped) atomicAdd(&s_flipped, flipped);
+        __syncthreads();
+        if (threadIdx.x == 0 && s_flipped) atomicAdd(&a.ctrl->scratch[1], (unsigned long long)s_flipped);
+        wolff_barrier(w, a.ctrl);
+    }
+    if (grower) wolff_call(w, last);
 }
 
 // ------------------------------------------------------------ sizes
@@ -1172,8 +1378,9 @@ struct ClusterDev {
     uint8_t *fresh = nullptr;
     int32_t *rank = nullptr;
     ClusterArgs::ChunkBase *chunk_base = nullptr;
-    uint32_t *stamp = nullptr;
-    int32_t *queue = nullptr;
+    WolffSync *wolff = nullptr;
+    unsigned wolff_grid = 0;
+    uint64_t wolff_launches = 0;
     unsigned long long *desc = nullptr;
     int64_t n_chunks = 0;
     int64_t n_tiles = 0;  // CTAs of the kernels that take a tile each
@@ -1206,8 +1413,6 @@ ClusterArgs cluster_args(plq_chain *c) {
     a.fresh = cd->fresh;
     a.rank = cd->rank;
     a.chunk_base = cd->chunk_base;
-    a.stamp = cd->stamp;
-    a.queue = cd->queue;
     a.g = c->g;
     a.q = c->q;
     a.extent = c->desc.extent;
@@ -1257,6 +1462,18 @@ struct TileKernels {
     static void apply_fresh(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
         apply_fresh_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
     }
+    static cudaError_t wolff(ClusterArgs a, WolffSync *w, uint32_t tiles, unsigned long long launch, unsigned grid,
+                             cudaStream_t st) {
+        void *params[] = {&a, &w, &tiles, &launch};
+        return cudaLaunchCooperativeKernel((const void *)wolff_kernel<D, SMALL>, dim3(grid), dim3(kThreads), params, 0, st);
+    }
+    // A CTA per tile and the growing one, as many as are resident together.
+    static cudaError_t wolff_grid(int64_t tiles, int sm_count, unsigned &grid) {
+        int per_sm = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wolff_kernel<D, SMALL>, kThreads, 0);
+        grid = (unsigned)std::min<int64_t>(tiles + 1, (int64_t)per_sm * sm_count);
+        return e != cudaSuccess || grid >= 2 ? e : cudaErrorLaunchOutOfResources;
+    }
     static void flatten(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
         flatten_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
     }
@@ -1269,13 +1486,16 @@ int sweep_t(plq_chain *c, uint64_t sweeps) {
     const int64_t n = c->n_sites;
     const unsigned gs = grid_stride_blocks(n);
     if (c->desc.extent == PLQ_EXTENT_SEEDED) {
-        ClusterArgs a = cluster_args(c);
-        a.updates = sweeps;
-        wolff_bfs_kernel<D><<<1, kBfsThreads, 0, c->stream>>>(a);
-        c->launches++;
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return plq_fail(PLQ_ECUDA, std::string("wolff launch: ") + cudaGetErrorString(e));
-        c->sweeps_done += sweeps;
+        for (uint64_t left = sweeps; left;) {
+            ClusterArgs a = cluster_args(c);
+            a.updates = std::min<uint64_t>(left, 1u << 30);
+            const cudaError_t e = K::wolff(a, cd->wolff, (uint32_t)cd->n_tiles, ++cd->wolff_launches, cd->wolff_grid,
+                                           c->stream);
+            c->launches++;
+            if (e != cudaSuccess) return plq_fail(PLQ_ECUDA, std::string("wolff launch: ") + cudaGetErrorString(e));
+            c->sweeps_done += a.updates;
+            left -= a.updates;
+        }
         cd->decomposed = false;
         return PLQ_OK;
     }
@@ -1365,6 +1585,26 @@ int cluster_validate(const plq_chain_desc *d) {
     return PLQ_OK;
 }
 
+template <int D>
+static cudaError_t wolff_grid_d(plq_chain *c, unsigned &grid) {
+    ClusterDev *cd = static_cast<ClusterDev *>(c->cl);
+    return cd->small_tiles ? TileKernels<D, true>::wolff_grid(cd->n_tiles, c->ctx->sm_count, grid)
+                           : TileKernels<D, D == 1>::wolff_grid(cd->n_tiles, c->ctx->sm_count, grid);
+}
+
+static cudaError_t wolff_grid(plq_chain *c, unsigned &grid) {
+    switch (c->d) {
+        case 1: return wolff_grid_d<1>(c, grid);
+        case 2: return wolff_grid_d<2>(c, grid);
+        case 3: return wolff_grid_d<3>(c, grid);
+        case 4: return wolff_grid_d<4>(c, grid);
+        case 5: return wolff_grid_d<5>(c, grid);
+        case 6: return wolff_grid_d<6>(c, grid);
+        case 7: return wolff_grid_d<7>(c, grid);
+        default: return wolff_grid_d<8>(c, grid);
+    }
+}
+
 int cluster_create(plq_chain *c) {
     ClusterDev *cd = new ClusterDev();
     c->cl = cd;
@@ -1404,9 +1644,11 @@ int cluster_create(plq_chain *c) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
     };
     if (c->desc.extent == PLQ_EXTENT_SEEDED) {
-        alloc((void **)&cd->stamp, sizeof(uint32_t) * (size_t)n);
-        alloc((void **)&cd->queue, sizeof(int32_t) * (size_t)n);
-        if (e == cudaSuccess) e = cudaMemsetAsync(cd->stamp, 0, sizeof(uint32_t) * (size_t)n, c->stream);
+        alloc((void **)&cd->wolff, sizeof(WolffSync));
+        if (e == cudaSuccess) e = cudaMemsetAsync(cd->wolff, 0, sizeof(WolffSync), c->stream);
+        if (e == cudaSuccess) e = wolff_grid(c, cd->wolff_grid);
+        alloc((void **)&cd->parent, sizeof(int32_t) * (size_t)n);
+        alloc((void **)&cd->local_root, sizeof(uint16_t) * tile_sites);
     } else {
         alloc((void **)&cd->bonds, (size_t)n);
         alloc((void **)&cd->parent, sizeof(int32_t) * (size_t)n);
@@ -1447,7 +1689,7 @@ int cluster_sweep(plq_chain *c) { return cluster_sweep_n(c, 1); }
 void cluster_free(plq_chain *c) {
     ClusterDev *cd = static_cast<ClusterDev *>(c->cl);
     if (!cd) return;
-    void *ptrs[] = {cd->bonds, cd->parent, cd->local_root, cd->fresh, cd->rank, cd->chunk_base, cd->stamp, cd->queue,
+    void *ptrs[] = {cd->bonds, cd->parent, cd->local_root, cd->fresh, cd->rank, cd->chunk_base, cd->wolff,
                     cd->desc, cd->events, cd->first_new, cd->sizes};
     for (void *p : ptrs)
         if (p) cudaFree(p);

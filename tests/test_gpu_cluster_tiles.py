@@ -72,3 +72,37 @@ def test_all_or_no_bonds(gpu, shape, beta):  # noqa: F811
                    plq.RNG_KEYED)
     next(chain)
     assert np.array_equal(chain.labels(), np.arange(n) if beta == 0.0 else np.zeros(n))
+
+
+WOLFF = [
+    (plq.ISING, 2, (31,), 1.0, plq.RELABEL_FORCED), (plq.ISING, 2, (2, 2), 0.4, plq.RELABEL_FORCED),
+    (plq.ISING, 2, (129, 17), 0.2, plq.RELABEL_FORCED),      # small clusters: growth alone
+    (plq.ISING, 2, (129, 17), 0.44, plq.RELABEL_REDRAW),     # ... ended after the call
+    (plq.POTTS, 3, (64, 96), 1.005, plq.RELABEL_FORCED),     # ... and the decomposition
+    (plq.ISING, 2, (33, 9, 5), 0.25, plq.RELABEL_FORCED), (plq.POTTS, 4, (34, 9, 5, 3), 0.5, plq.RELABEL_REDRAW),
+    (plq.ISING, 2, (33, 9, 5), 50.0, plq.RELABEL_FORCED), (plq.ISING, 2, (33, 9, 5), 0.0, plq.RELABEL_FORCED),
+    (plq.ISING, 2, (401, 307), 0.47, plq.RELABEL_FORCED),
+]
+
+
+@pytest.mark.parametrize("case", WOLFF, ids=lambda c: f"{c[0]}-{c[1]}-{'x'.join(map(str, c[2]))}-{c[3]}-{c[4]}")
+def test_wolff(oracle, gpu, case):  # noqa: F811
+    """Growth alone, growth that ends after the call and the decomposition give the seeded filter's
+    states and cluster size, one update a launch and many in one."""
+    kind, q, shape, beta, relabel = case
+    lat = oracle.Lattice(shape)
+    model = _model(oracle, kind, q)
+    start, _ = plq.hot_start(12, q, lat.n_sites)
+    args = (gpu, kind, q, shape, plq.EXTENT_SEEDED, relabel, beta, 12, start, plq.RNG_KEYED)
+    one, many = _chain(*args), _chain(*args)
+    updates = 12
+    many.advance(updates)
+    want = start.copy()
+    for t in range(updates):
+        before = want.copy()
+        oracle.keyed_cluster_sweep(model, lat, want, oracle.SEEDED, relabel, beta, oracle.fold_seed(12), t)
+        assert np.array_equal(next(one), want), t
+        if relabel == plq.RELABEL_FORCED:
+            flipped = int((before != want).sum())
+            assert one.size_histogram()[flipped.bit_length() - 1] == 1
+    assert np.array_equal(many.read(), want)
