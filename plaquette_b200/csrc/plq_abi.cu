@@ -240,7 +240,8 @@ void chain_free(plq_chain *c) {
     cluster_free(c);
     void *ptrs[] = {c->d_state, c->d_state_alt, c->d_io, c->d_hb53, c->d_hb24, c->d_metro53, c->d_metro24,
                     c->d_jump, c->d_ctrl, c->d_desc, c->d_obs, c->d_snap, c->d_snap_obs, c->d_loop_bits,
-                    c->d_meas, c->d_pairs, c->d_hb53_fused, c->d_packed, c->d_first_hash};
+                    c->d_meas, c->d_pairs, c->d_hb53_fused, c->d_packed, c->d_first_hash,
+                    c->d_resident};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
@@ -326,6 +327,24 @@ int32_t first_bad_start(int32_t n, const uint8_t *const *starts, const int64_t *
         return starts[k] && first_state_at_least_serial(starts[k], n_vars[k], q[k]) >= 0;
     });
     return (int32_t)m;
+}
+
+// The lattices that run resident: where a barrier is cheaper than a launch and
+// the body at least as fast as the per-pass kernel's.
+//  * packed kinds: always (250^3 Ising, whose rows are no multiple of 64 sites, 124 -> 33 us
+//    a sweep), but for rows of whole 64-site words from 2^23 sites on, where the passes that
+//    stream each site's first hash from memory win (256^3: 25.0 us a sweep against 27.2;
+//    4096 x 2048: 16.7 against 16.1);
+//  * one keyed site per thread: always;
+//  * words and ranks: up to one wave of CTAs (400 x 400 x 100 Potts on the PCG stream, several
+//    waves: 131 us a sweep resident, 111 with a launch per pass).
+static bool resident_wanted(const ResidentPlan &p, int64_t n_sites, bool whole_words) {
+    switch (p.kind) {
+        case ResidentKind::kSites: return !(whole_words && n_sites >= (int64_t(1) << 23));
+        case ResidentKind::kWords:
+        case ResidentKind::kGeneric: return p.chunks <= p.grid;
+        default: return p.kind != ResidentKind::kNone;
+    }
 }
 
 extern "C" int plq_chain_create(plq_ctx *ctx, const plq_chain_desc *desc, const uint8_t *start,
@@ -461,9 +480,26 @@ extern "C" int plq_chain_create(plq_ctx *ctx, const plq_chain_desc *desc, const 
                 hb53_shifted.push_back(cut << 11);
             }
         }
-        if (!(desc->flags & (PLQ_FLAG_NO_FUSED | PLQ_FLAG_GENERIC_PASS | PLQ_FLAG_NO_PACKED)) && !c->link &&
-            packed_chain_eligible(desc->model, c->q, c->d, c->g.L, desc->updater, desc->rng)) {
-            c->packed = true;
+        c->packed = !(desc->flags & (PLQ_FLAG_NO_FUSED | PLQ_FLAG_GENERIC_PASS | PLQ_FLAG_NO_PACKED)) && !c->link &&
+                    packed_chain_eligible(desc->model, c->q, c->d, c->g.L, desc->updater, desc->rng);
+        const bool wants_fused = !c->packed && !(desc->flags & PLQ_FLAG_NO_FUSED) &&
+                                 fused3d_eligible(desc->model, c->q, c->d, c->g.L, desc->updater, desc->rng) &&
+                                 table_bytes <= (size_t)fused3d_table_limit_bytes() && shifted_ok;
+        if (!c->lookback && !wants_fused && !(desc->flags & (PLQ_FLAG_NO_FUSED | PLQ_FLAG_GENERIC_PASS | PLQ_FLAG_NO_PACKED |
+                                                          PLQ_FLAG_NO_FIRST_HASH))) {
+            const ResidentKind kind = resident_kind(desc->model, c->q, c->d, c->g.L, desc->updater, desc->rng, c->words);
+            ResidentPlan plan;
+            if (kind != ResidentKind::kNone) {
+                e = resident_plan(kind, c->g, desc->rng == PLQ_RNG_STREAM, c->ctx->sm_count, plan);
+                if (e != cudaSuccess) return fail(cuda_fail(e, "resident launch plan"));
+            }
+            if (resident_wanted(plan, c->n_sites, c->packed)) {
+                c->resident = plan;
+                if (plan.packed_bytes) e = cudaMalloc(&c->d_resident, plan.packed_bytes);
+                if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc(resident words)"));
+            }
+        }
+        if (c->packed && c->resident.kind == ResidentKind::kNone) {
             e = cudaMalloc((void **)&c->d_packed, (size_t)(c->n_sites / 64) * sizeof(uint64_t));
             if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc(packed state)"));
             // every site's sweep-independent first keyed round lowbias32_head(seed ^ site) (4 B/site):
@@ -485,9 +521,7 @@ extern "C" int plq_chain_create(plq_ctx *ctx, const plq_chain_desc *desc, const 
                 }
             }
         }
-        if (!c->packed && !(desc->flags & PLQ_FLAG_NO_FUSED) &&
-            fused3d_eligible(desc->model, c->q, c->d, c->g.L, desc->updater, desc->rng) &&
-            table_bytes <= (size_t)fused3d_table_limit_bytes() && shifted_ok) {
+        if (wants_fused) {
             c->fused = true;
             if (!hb53_shifted.empty()) {
                 int r3 = upload(hb53_shifted, &c->d_hb53_fused, c->stream);
@@ -610,6 +644,36 @@ static int fused_sweep(plq_chain *c) {
     return PLQ_OK;
 }
 
+// `samples` times `sweeps` sweeps in one launch, each followed by a snapshot
+// and a measurement where there is a place for them.
+static int resident_sweeps(plq_chain *c, uint64_t samples, uint64_t sweeps, uint8_t *snapshots, long long *primaries) {
+    if (!samples || (!sweeps && !snapshots && !primaries)) return PLQ_OK;
+    ResidentArgs r;
+    std::memset(&r, 0, sizeof r);
+    r.p = local_args(c);
+    r.p.sweep32 = (uint32_t)c->sweeps_done;
+    r.p.pass_offset = c->host_pos;
+    r.n_vars = c->n_vars;
+    r.samples = samples;
+    r.sweeps = sweeps;
+    r.snapshots = snapshots;
+    r.primaries = primaries;
+    r.n_primaries = primaries_count(c->desc.model, c->q);
+    r.packed = c->d_resident;
+    if (primaries)
+        PLQ_CUDA(cudaMemsetAsync(primaries, 0, sizeof(long long) * (size_t)(samples * (uint64_t)r.n_primaries), c->stream),
+                 "primaries clear");
+    r.arrived = c->resident_arrivals;
+    PLQ_CUDA(launch_resident(c->resident, r, c->stream), "resident launch");
+    if (!c->resident.cluster)
+        c->resident_arrivals += c->resident.grid * resident_barriers(c->resident, c->link ? 2 * c->d : 2, samples, sweeps,
+                                                                     snapshots || primaries);
+    c->launches++;
+    if (c->desc.rng == PLQ_RNG_STREAM) c->host_pos += samples * sweeps * (uint64_t)c->n_vars;
+    c->sweeps_done += samples * sweeps;
+    return PLQ_OK;
+}
+
 // `sweeps` sweeps of a packed chain: the bytes packed once, two colour passes
 // per sweep on the words (the keyed sweep index as the byte passes use it),
 // the words unpacked at the end.
@@ -708,6 +772,7 @@ int local_sweep(plq_chain *c) {
 
 static int run_sweeps(plq_chain *c, uint64_t sweeps) {
     if (c->cluster) return sweeps ? cluster_sweep_n(c, sweeps) : PLQ_OK;
+    if (c->resident.kind != ResidentKind::kNone) return resident_sweeps(c, 1, sweeps, nullptr, nullptr);
     if (c->packed) return packed_sweeps(c, sweeps);
     for (uint64_t t = 0; t < sweeps; ++t) {
         int rc = c->cluster ? cluster_sweep(c) : local_sweep(c);
@@ -934,7 +999,12 @@ extern "C" int plq_chain_next_batch(plq_chain *c, int64_t count, uint8_t *out_st
     int64_t done = 0;
     while (done < count) {
         int64_t m = std::min<int64_t>(cap, count - done);
-        for (int64_t k = 0; k < m; ++k) {
+        if (c->resident.kind != ResidentKind::kNone) {
+            int rc = resident_sweeps(c, (uint64_t)m, (uint64_t)c->desc.sweeps_between, out_states ? c->d_snap : nullptr,
+                                     out_primaries ? c->d_snap_obs : nullptr);
+            if (rc != PLQ_OK) return rc;
+        }
+        for (int64_t k = 0; k < (c->resident.kind != ResidentKind::kNone ? 0 : m); ++k) {
             int rc = run_sweeps(c, (uint64_t)c->desc.sweeps_between);
             if (rc != PLQ_OK) return rc;
             if (out_states) {

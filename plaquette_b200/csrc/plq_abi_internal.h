@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/plaquette.h"
+#include "plq_resident.h"
 #include "plq_device.cuh"
 #include "plq_fused.h"
 #include "plq_tables.h"
@@ -48,6 +49,9 @@ struct plq_chain {
     bool packed = false;          // q = 2 keyed sites: sweeps on a bit-packed copy (plq_packed3d.cu)
     uint64_t *d_packed = nullptr; // n_sites / 64 words
     void *d_first_hash = nullptr; // packed chains: lowbias32_head(seed ^ site) of every site (plq_packed3d.cu)
+    plq::ResidentPlan resident;  // the sweeps of a call in one launch (plq_resident.cu)
+    void *d_resident = nullptr;   // ... their packed words
+    uint64_t resident_arrivals = 0;  // ... arrivals at their grid barrier in all launches
     int fused_tz = 0;
     plq::FusedMaps fused_maps[2];          // TMA descriptors of the two state buffers
     const uint8_t *fused_map_buf[2] = {nullptr, nullptr};

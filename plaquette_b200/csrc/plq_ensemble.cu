@@ -38,6 +38,7 @@
 #include "plq_abi_internal.h"
 #include "plq_device.cuh"
 #include "plq_geom.cuh"
+#include "plq_items.cuh"
 #include "plq_local.h"
 #include "plq_local_impl.cuh"
 #include "plq_packed.cuh"
@@ -187,233 +188,6 @@ __device__ void grid_barrier(const EnsArgs &e) {
         __threadfence();
     }
     __syncthreads();
-}
-
-template <int D>
-__device__ void run_words(const LocalArgs &a, int link, int64_t chunk, int R) {
-    const bool st = a.jump != nullptr;
-    if (link) {
-        if (D >= 2) {
-            if (st) link_words_chunk<D, true>(a, chunk, R);
-            else link_words_chunk<D, false>(a, chunk, R);
-        }
-    } else if (a.q == 3) {
-        if (st) site_words_chunk<D, 3, true>(a, chunk, R);
-        else site_words_chunk<D, 3, false>(a, chunk, R);
-    } else if (a.q == 4) {
-        if (st) site_words_chunk<D, 4, true>(a, chunk, R);
-        else site_words_chunk<D, 4, false>(a, chunk, R);
-    } else {
-        if (st) site_words_chunk<D, 2, true>(a, chunk, R);
-        else site_words_chunk<D, 2, false>(a, chunk, R);
-    }
-}
-
-// WORDS_ONLY: every member runs four sites at a time, so the generic body is
-// compiled out (far fewer registers, more CTAs per SM).
-template <int R, bool WORDS_ONLY>
-__device__ void run_item(const LocalArgs &a, int d, int link, int64_t chunk, int wpt) {
-    if (WORDS_ONLY || a.words) {
-        switch (d) {
-            case 1: run_words<1>(a, link, chunk, wpt); break;
-            case 2: run_words<2>(a, link, chunk, wpt); break;
-            case 3: run_words<3>(a, link, chunk, wpt); break;
-            case 4: run_words<4>(a, link, chunk, wpt); break;
-            default: break;
-        }
-        return;
-    }
-    if (WORDS_ONLY) return;
-    if (link) {
-        switch (d) {
-            case 2: local_chunk<2, true, false, R>(a, chunk); break;
-            case 3: local_chunk<3, true, false, R>(a, chunk); break;
-            case 4: local_chunk<4, true, false, R>(a, chunk); break;
-            default: break;
-        }
-    } else {
-        switch (d) {
-            case 1: local_chunk<1, false, false, R>(a, chunk); break;
-            case 2: local_chunk<2, false, false, R>(a, chunk); break;
-            case 3: local_chunk<3, false, false, R>(a, chunk); break;
-            case 4: local_chunk<4, false, false, R>(a, chunk); break;
-            default: break;
-        }
-    }
-}
-
-// ---- Z2 gauge members with L0 <= 32 on the keyed stream: links bit-packed by rows.
-// Inside a persistent launch such a member's links live in pk: word dir * rows + r
-// holds bit x = U_dir(x, r) for row r (the site index over directions >= 1).  A
-// work item takes rows of one (direction mu, parity) pass: the six staples of
-// every link of a row come out of XORs of whole row words (a shift along
-// direction 0 is a rotation of the row, along the others another row), their
-// count of unsatisfied staples out of a bit-sliced counter, and each link of
-// the pass's parity then decides exactly as the byte body does -- the same key
-// cur + 4(d-1) - 2 * unsatisfied, the same keyed draw of variable site * d + mu,
-// the same table -- so results are bit-identical.  The launch packs the bytes
-// first and unpacks them at its end (pack_links_kernel).
-
-// Rows of a lattice (sites over directions >= 1): L1 * L2 * ... (extents past
-// d are 1), by multiplication.
-__host__ __device__ __forceinline__ uint32_t row_count(const Geom &g) {
-    uint32_t n = 1;
-#pragma unroll
-    for (int k = 1; k < kMaxD; ++k) n *= (uint32_t)g.L[k];
-    return n;
-}
-
-// Row r's coordinates along directions 1..D-1: their parity and the row
-// offsets to the +k / -k neighbour rows (periodic).  The row stride of
-// direction k is L1 * ... * L(k-1).
-template <int D>
-__device__ __forceinline__ int row_geometry(const Geom &g, uint32_t r, int32_t *op, int32_t *om) {
-    uint32_t rr = r;
-    int par = 0;
-    int32_t rs = 1;
-#pragma unroll
-    for (int k = 1; k < D; ++k) {
-        const uint32_t q = fdiv(rr, g.dm[k], g.dl[k]);
-        const int32_t c = (int32_t)(rr - q * (uint32_t)g.L[k]);
-        rr = q;
-        par += c;
-        op[k] = c + 1 < g.L[k] ? rs : -(g.L[k] - 1) * rs;
-        om[k] = c > 0 ? -rs : (g.L[k] - 1) * rs;
-        rs *= g.L[k];
-    }
-    return par;
-}
-
-// q = 2 sites (Ising, or Potts at q = 2) packed by rows: the per-site count of
-// neighbours in state 1 comes out of the bit-sliced counter over the 2d
-// neighbour rows (d <= 3: at most 6), key cur + 2 * count as the byte body's.
-template <int D, class W>
-__device__ void packed_site_item(const LocalArgs &a, W *pk, int64_t chunk, int R, const uint2 *tab) {
-    const uint32_t L0 = (uint32_t)a.g.L[0];
-    const uint32_t rows = row_count(a.g);
-    const W full = L0 == 8 * sizeof(W) ? ~(W)0 : (((W)1 << L0) - 1);
-    const uint32_t r0 = (uint32_t)(chunk * (int64_t)blockDim.x * R) + threadIdx.x * (uint32_t)R;
-    const bool hb = a.kernel == PLQ_HEATBATH;
-    const uint32_t sweep_mix = keyed_mix(a.sweep32);
-#pragma unroll 1
-    for (int i = 0; i < R; ++i) {
-        const uint32_t r = r0 + (uint32_t)i;
-        if (r >= rows) break;
-        int32_t op[4] = {0, 0, 0, 0}, om[4] = {0, 0, 0, 0};
-        const int par = row_geometry<D>(a.g, r, op, om);
-        const W C = pk[r];
-        W c0 = 0, c1 = 0, c2 = 0;
-        count_add(c0, c1, c2, row_xp(C, L0, full));
-        count_add(c0, c1, c2, row_xm(C, L0, full));
-#pragma unroll
-        for (int k = 1; k < D; ++k) {
-            count_add(c0, c1, c2, pk[r + (uint32_t)op[k]]);
-            count_add(c0, c1, c2, pk[r + (uint32_t)om[k]]);
-        }
-        const uint32_t x0 = (uint32_t)((a.color ^ par) & 1);
-        const int n = (int)(L0 / 2);
-        const uint32_t v0 = r * L0 + x0;  // the keyed stream's index of the row's first variable
-        const W flip = hb ? decide_row<W, 2, true>(C >> x0, c0 >> x0, c1 >> x0, c2 >> x0, n, v0, a.seed32, sweep_mix, tab)
-                          : decide_row<W, 2, false>(C >> x0, c0 >> x0, c1 >> x0, c2 >> x0, n, v0, a.seed32, sweep_mix, tab);
-        pk[r] = C ^ (flip << x0);
-    }
-}
-
-// Energy integer of packed rows [c * blockDim, (c + 1) * blockDim), one row per
-// thread: sites -- the bond sum (Ising) or agreement count (Potts) over the
-// +mu bonds; links -- the plaquette sum over mu < nu (as energy_chunk).
-template <int D, class W>
-__device__ long long packed_energy_rows(const LocalArgs &a, const W *pk, int link, int64_t c) {
-    const uint32_t L0 = (uint32_t)a.g.L[0];
-    const uint32_t rows = row_count(a.g);
-    const W full = L0 == 8 * sizeof(W) ? ~(W)0 : (((W)1 << L0) - 1);
-    const uint32_t r = (uint32_t)(c * (int64_t)blockDim.x) + threadIdx.x;
-    if (r >= rows) return 0;
-    int32_t op[4] = {0, 0, 0, 0}, om[4] = {0, 0, 0, 0};
-    row_geometry<D>(a.g, r, op, om);
-    long long acc = 0;
-    if (!link) {
-        const W C = pk[r];
-        int diff = popc_w((C ^ row_xp(C, L0, full)) & full);
-        long long pairs = L0;
-#pragma unroll
-        for (int k = 1; k < D; ++k) {
-            diff += popc_w(C ^ pk[r + (uint32_t)op[k]]);
-            pairs += L0;
-        }
-        acc = a.model == PLQ_ISING ? pairs - 2ll * diff : pairs - diff;
-    } else {
-#pragma unroll
-        for (int mu = 0; mu < D; ++mu) {
-#pragma unroll
-            for (int nu = mu + 1; nu < D; ++nu) {
-                const W *Pmu = pk + (uint32_t)mu * rows, *Pnu = pk + (uint32_t)nu * rows;
-                const W umu = Pmu[r], unu = Pnu[r];
-                // U_nu(s + mu): mu = 0 a rotation of the row, else the +mu row
-                const W nu_smu = mu == 0 ? row_xp(unu, L0, full) : Pnu[r + (uint32_t)op[mu]];
-                const W mu_snu = Pmu[r + (uint32_t)op[nu]];  // nu >= 1
-                acc += (long long)L0 - 2ll * popc_w(umu ^ nu_smu ^ mu_snu ^ unu);
-            }
-        }
-    }
-    return acc;
-}
-
-// MU: the pass's direction (a compile-time constant, so the staple terms that
-// are row rotations and those that are other rows are fixed per variant).
-template <int D, int MU>
-__device__ void packed_link_item(const LocalArgs &a, uint32_t *pk, int64_t chunk, int R, const uint2 *tab) {
-    // (rows of at most 32 links)
-    const uint32_t L0 = (uint32_t)a.g.L[0];
-    const uint32_t rows = row_count(a.g);
-    constexpr int mu = MU;
-    const uint32_t full = L0 == 32 ? 0xFFFFFFFFu : ((1u << L0) - 1u);
-    const uint32_t r0 = (uint32_t)(chunk * (int64_t)blockDim.x * R) + threadIdx.x * (uint32_t)R;
-    const bool hb = a.kernel == PLQ_HEATBATH;
-    const uint32_t sweep_mix = keyed_mix(a.sweep32);
-#pragma unroll 1
-    for (int i = 0; i < R; ++i) {
-        const uint32_t r = r0 + (uint32_t)i;
-        if (r >= rows) break;
-        int32_t op[4] = {0, 0, 0, 0}, om[4] = {0, 0, 0, 0};
-        const int par = row_geometry<D>(a.g, r, op, om);
-        const int32_t op_mu = mu > 0 ? op[mu] : 0;
-        const uint32_t Umu = pk[(uint32_t)mu * rows + r];
-        uint32_t c0 = 0, c1 = 0, c2 = 0;  // satisfied staples per link
-#pragma unroll
-        for (int nu = 0; nu < D; ++nu) {
-            if (nu == mu) continue;
-            const uint32_t *Pnu = pk + (uint32_t)nu * rows;
-            const uint32_t *Pmu = pk + (uint32_t)mu * rows;
-            // forward: U_nu(s+mu) U_mu(s+nu) U_nu(s)
-            const uint32_t nu_s = Pnu[r];
-            const uint32_t nu_smu = mu == 0 ? row_xp(nu_s, L0, full) : Pnu[r + (uint32_t)op_mu];
-            const uint32_t mu_snu = nu == 0 ? row_xp(Umu, L0, full) : Pmu[r + (uint32_t)op[nu]];
-            count_add(c0, c1, c2, ~(nu_smu ^ mu_snu ^ nu_s));
-            // backward: U_nu(s+mu-nu) U_mu(s-nu) U_nu(s-nu)
-            uint32_t nu_smn, mu_smn, nu_smumn;
-            if (nu == 0) {
-                nu_smn = row_xm(nu_s, L0, full);
-                mu_smn = row_xm(Umu, L0, full);
-                nu_smumn = row_xm(nu_smu, L0, full);
-            } else {
-                nu_smn = Pnu[r + (uint32_t)om[nu]];
-                mu_smn = Pmu[r + (uint32_t)om[nu]];
-                nu_smumn = mu == 0 ? row_xp(nu_smn, L0, full) : Pnu[r + (uint32_t)op_mu + (uint32_t)om[nu]];
-            }
-            count_add(c0, c1, c2, ~(nu_smumn ^ mu_smn ^ nu_smn));
-        }
-        // the links of the pass's parity: x with (x + par) % 2 == colour; the byte body's key
-        // cur + 4(d-1) - 2 * unsatisfied is cur + 2 * satisfied
-        const uint32_t x0 = (uint32_t)((a.color ^ par) & 1);
-        const int n = (int)(L0 / 2);
-        const uint32_t v0 = (r * L0 + x0) * (uint32_t)D + (uint32_t)mu;  // keyed index of link (x0, r, mu)
-        const uint32_t flip = hb ? decide_row<uint32_t, 2 * D, true>(Umu >> x0, c0 >> x0, c1 >> x0, c2 >> x0, n, v0,
-                                                                     a.seed32, sweep_mix, tab)
-                                 : decide_row<uint32_t, 2 * D, false>(Umu >> x0, c0 >> x0, c1 >> x0, c2 >> x0, n, v0,
-                                                                      a.seed32, sweep_mix, tab);
-        pk[(uint32_t)mu * rows + r] = Umu ^ (flip << x0);
-    }
 }
 
 // Packing entry of one member: its rows (of all d directions, for links)

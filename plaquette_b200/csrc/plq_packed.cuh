@@ -149,6 +149,27 @@ __device__ __forceinline__ uint32_t key_word(W P, W Q, int c) {
     return x;
 }
 
+// Group c of a row alone: its variables 8c .. 8c + 7 (those below n), the flips
+// at 2i of 16 bits.  Rows as decide_row's.  HEADS: the variables' first rounds
+// are given (h1, any value past n).
+template <class W, int DV, bool HB, bool HEADS>
+__device__ __forceinline__ uint32_t decide_group(W Cs, W c0s, W c1s, W c2s, int c, int n, uint32_t v0, uint32_t seed32,
+                                                 uint32_t mix, const uint2 *tab, const uint32_t (&h1)[8]) {
+    const W M = (W)0x5555555555555555ull;
+    const W P = (Cs & M) | ((c0s << 1) & ~M);
+    const W Q = (c1s & M) | ((c2s << 1) & ~M);
+    const char *tb = reinterpret_cast<const char *>(tab);
+    const uint32_t x = key_word(P, Q, c), vc = v0 + (uint32_t)(8 * c * DV);
+    const int m = n - 8 * c < 8 ? n - 8 * c : 8;
+    const uint32_t valid = 0x5555u & ((1u << (2 * m)) - 1u);
+    uint32_t out;
+    if (tab[kTableEntries].x) out = decide8_marked<DV, HB>(x, m, vc, seed32, mix, tb);
+    else if (HEADS) out = decide8_h1<HB>(x, h1, mix, tb);
+    else out = decide8<DV, HB, false>(x, 8, vc, seed32, mix, tb);
+    if (HB) out ^= (uint32_t)(P >> (16 * c));  // new states -> flips
+    return out & valid;
+}
+
 template <class W, int DV, bool HB>
 __device__ __forceinline__ W decide_row(W Cs, W c0s, W c1s, W c2s, int n, uint32_t v0, uint32_t seed32,
                                         uint32_t mix, const uint2 *tab) {
