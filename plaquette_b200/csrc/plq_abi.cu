@@ -485,17 +485,25 @@ extern "C" int plq_chain_create(plq_ctx *ctx, const plq_chain_desc *desc, const 
         const bool wants_fused = !c->packed && !(desc->flags & PLQ_FLAG_NO_FUSED) &&
                                  fused3d_eligible(desc->model, c->q, c->d, c->g.L, desc->updater, desc->rng) &&
                                  table_bytes <= (size_t)fused3d_table_limit_bytes() && shifted_ok;
-        if (!c->lookback && !wants_fused && !(desc->flags & (PLQ_FLAG_NO_FUSED | PLQ_FLAG_GENERIC_PASS | PLQ_FLAG_NO_PACKED |
+        // a packed kind's cut points on the stream are compared shifted left by 11 with whole draws
+        bool cuts_below = true;
+        for (const std::vector<uint64_t> *cuts : {&t.metro53, &t.hb53})
+            for (uint64_t cut : *cuts) cuts_below = cuts_below && (cut == ~0ull || cut < (uint64_t(1) << 53));
+        if (!wants_fused && !(desc->flags & (PLQ_FLAG_NO_FUSED | PLQ_FLAG_GENERIC_PASS | PLQ_FLAG_NO_PACKED |
                                                           PLQ_FLAG_NO_FIRST_HASH))) {
             const ResidentKind kind = resident_kind(desc->model, c->q, c->d, c->g.L, desc->updater, desc->rng, c->words);
+            const bool packed_kind = kind == ResidentKind::kSites || kind == ResidentKind::kLinks32 || kind == ResidentKind::kLinks64;
             ResidentPlan plan;
-            if (kind != ResidentKind::kNone) {
-                e = resident_plan(kind, c->g, desc->rng == PLQ_RNG_STREAM, c->ctx->sm_count, plan);
+            if (kind != ResidentKind::kNone && (cuts_below || desc->rng != PLQ_RNG_STREAM || !packed_kind)) {
+                e = resident_plan(kind, c->g, desc->rng == PLQ_RNG_STREAM, desc->updater == PLQ_HEATBATH, c->ctx->sm_count,
+                                  plan);
                 if (e != cudaSuccess) return fail(cuda_fail(e, "resident launch plan"));
             }
             if (resident_wanted(plan, c->n_sites, c->packed)) {
                 c->resident = plan;
-                if (plan.packed_bytes) e = cudaMalloc(&c->d_resident, plan.packed_bytes);
+                c->resident_totals = (plan.packed_bytes + 15) & ~(size_t)15;
+                if (plan.packed_bytes)
+                    e = cudaMalloc(&c->d_resident, c->resident_totals + (plan.stream_draws ? kResidentTotals * sizeof(uint32_t) : 0));
                 if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc(resident words)"));
             }
         }
@@ -541,7 +549,7 @@ extern "C" int plq_chain_create(plq_ctx *ctx, const plq_chain_desc *desc, const 
                 e = cudaEventCreateWithFlags(&c->measured[k], cudaEventDisableTiming);
             if (e != cudaSuccess) return fail(cuda_fail(e, "measurement stream"));
         }
-        if (c->lookback) {
+        if (c->lookback && c->resident.kind == ResidentKind::kNone) {
             c->n_chunks = local_chunks(n);
             // descriptors for the larger chunk count of the two look-back pass kernels
             const int64_t n_desc = std::max<int64_t>(c->n_chunks, scan_chunks(n));
@@ -660,6 +668,8 @@ static int resident_sweeps(plq_chain *c, uint64_t samples, uint64_t sweeps, uint
     r.primaries = primaries;
     r.n_primaries = primaries_count(c->desc.model, c->q);
     r.packed = c->d_resident;
+    r.totals = reinterpret_cast<uint32_t *>(static_cast<uint8_t *>(c->d_resident) + c->resident_totals);
+    r.p.pos_in = (int)(c->lookback_passes & 1);  // (the launch leaves the position where it found it)
     if (primaries)
         PLQ_CUDA(cudaMemsetAsync(primaries, 0, sizeof(long long) * (size_t)(samples * (uint64_t)r.n_primaries), c->stream),
                  "primaries clear");
@@ -669,7 +679,7 @@ static int resident_sweeps(plq_chain *c, uint64_t samples, uint64_t sweeps, uint
         c->resident_arrivals += c->resident.grid * resident_barriers(c->resident, c->link ? 2 * c->d : 2, samples, sweeps,
                                                                      snapshots || primaries);
     c->launches++;
-    if (c->desc.rng == PLQ_RNG_STREAM) c->host_pos += samples * sweeps * (uint64_t)c->n_vars;
+    if (c->desc.rng == PLQ_RNG_STREAM && !c->lookback) c->host_pos += samples * sweeps * (uint64_t)c->n_vars;
     c->sweeps_done += samples * sweeps;
     return PLQ_OK;
 }

@@ -51,6 +51,7 @@ struct plq_chain {
     void *d_first_hash = nullptr; // packed chains: lowbias32_head(seed ^ site) of every site (plq_packed3d.cu)
     plq::ResidentPlan resident;  // the sweeps of a call in one launch (plq_resident.cu)
     void *d_resident = nullptr;   // ... their packed words
+    size_t resident_totals = 0;   // ... where their CTAs' draw totals lie behind them
     uint64_t resident_arrivals = 0;  // ... arrivals at their grid barrier in all launches
     int fused_tz = 0;
     plq::FusedMaps fused_maps[2];          // TMA descriptors of the two state buffers

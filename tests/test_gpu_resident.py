@@ -119,3 +119,24 @@ def test_chains_of_several_threads(gpu):
     for a, b in pairs:
         b.advance(100)
         assert np.array_equal(a.read(), b.read())
+
+
+@pytest.mark.parametrize("kernel", [plq.METROPOLIS, plq.HEATBATH], ids=["metro", "hb"])
+@pytest.mark.parametrize("shape", SITES + [(256, 250), (512, 190, 40)], ids=lambda s: "x".join(map(str, s)))
+def test_stream_sites(gpu, shape, kernel):
+    beta = 0.44 if len(shape) == 2 else 0.22
+    _check(*_pair(gpu, plq.ISING, 2, shape, kernel, plq.RNG_STREAM, beta, h=0.1, sweeps_between=2))
+
+
+@pytest.mark.parametrize("kernel", [plq.METROPOLIS, plq.HEATBATH], ids=["metro", "hb"])
+@pytest.mark.parametrize("shape", LINKS, ids=lambda s: "x".join(map(str, s)))
+def test_stream_links(gpu, shape, kernel):
+    _check(*_pair(gpu, plq.GAUGE, 2, shape, kernel, plq.RNG_STREAM, {2: 0.7, 3: 0.76, 4: 0.44}[len(shape)],
+                  sweeps_between=2))
+
+
+@pytest.mark.parametrize("beta", [0.0, 0.7, 300.0])
+@pytest.mark.parametrize("shape", [(8, 6), (66, 12), (130, 60, 22)], ids=lambda s: "x".join(map(str, s)))
+def test_stream_extreme_couplings(gpu, shape, beta):
+    """No variable draws (beta = 0: every move is downhill), probabilities of 0 (cut points of 0)."""
+    _check(*_pair(gpu, plq.POTTS, 2, shape, plq.METROPOLIS, plq.RNG_STREAM, beta, sweeps_between=1))
