@@ -241,7 +241,7 @@ void chain_free(plq_chain *c) {
     void *ptrs[] = {c->d_state, c->d_state_alt, c->d_io, c->d_hb53, c->d_hb24, c->d_metro53, c->d_metro24,
                     c->d_jump, c->d_ctrl, c->d_desc, c->d_obs, c->d_snap, c->d_snap_obs, c->d_loop_bits,
                     c->d_meas, c->d_pairs, c->d_hb53_fused, c->d_packed, c->d_first_hash,
-                    c->d_resident};
+                    c->d_resident, c->d_pair_words};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
@@ -881,11 +881,17 @@ extern "C" int plq_chain_axis_pair_sums(plq_chain *c, int64_t *out, int64_t capa
     pairs.insert(pairs.end(), rs.begin(), rs.end());
     std::vector<long long> differ(n_pairs, 0);
     if (n_pairs) {
-        PLQ_CUDA(cudaMemcpyAsync(c->d_pairs, pairs.data(), sizeof(int32_t) * 2 * (size_t)n_pairs,
-                                 cudaMemcpyHostToDevice, c->stream),
-                 "pair lists");
-        cudaError_t e = launch_pair_differ(c->d_state, c->g, c->d_pairs, c->d_pairs + n_pairs, n_pairs, c->d_meas,
-                                           c->stream);
+        cudaError_t e;
+        const size_t words = pair_words_bytes(c->g, c->q);
+        if (words) {
+            if (!c->d_pair_words) PLQ_CUDA(cudaMalloc((void **)&c->d_pair_words, words), "cudaMalloc(pair words)");
+            e = launch_pair_bits(c->d_state, c->g, c->q, c->d_pair_words, n_pairs, c->d_meas, c->ctx->sm_count, c->stream);
+        } else {
+            PLQ_CUDA(cudaMemcpyAsync(c->d_pairs, pairs.data(), sizeof(int32_t) * 2 * (size_t)n_pairs,
+                                     cudaMemcpyHostToDevice, c->stream),
+                     "pair lists");
+            e = launch_pair_differ(c->d_state, c->g, c->d_pairs, c->d_pairs + n_pairs, n_pairs, c->d_meas, c->stream);
+        }
         c->launches++;
         if (e != cudaSuccess) return cuda_fail(e, "pair sums");
         PLQ_CUDA(cudaMemcpyAsync(differ.data(), c->d_meas, sizeof(long long) * (size_t)n_pairs,

@@ -76,6 +76,7 @@ struct plq_chain {
     long long *d_obs = nullptr;
     uint8_t *d_snap = nullptr;
     uint32_t *d_loop_bits = nullptr;   // Wilson line parities (n_sites * d words), on first use
+    uint64_t *d_pair_words = nullptr;  // the correlator's bit planes, on first use
     long long *d_meas = nullptr;       // measurement results (meas_cap int64)
     int32_t *d_pairs = nullptr;        // (mu, r) pair lists of the correlator (2 * meas_cap)
     int64_t meas_cap = 0;

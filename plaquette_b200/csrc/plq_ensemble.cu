@@ -110,10 +110,14 @@ ShapeKey shape_key(const plq_chain_desc &d) {
     return k;
 }
 
-int tuned_wpt(const plq_chain_desc &d) {
+// Packed members start at one row a thread: a row is eight and more decisions,
+// and the tuner chose one for every shape of the workloads (256 tempered Ising
+// replicas of 16^3 to 64^3 beside 64 gauge lattices of 8^4 to 24^4: 148 us a sweep
+// at four, @@WPT at one).
+int tuned_wpt(const plq_chain_desc &d, bool packed) {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tuned.find(shape_key(d));
-    return it == g_tuned.end() ? kWordsPerThread : it->second.wpt;
+    return it == g_tuned.end() ? (packed ? 1 : kWordsPerThread) : it->second.wpt;
 }
 
 // Device-resident launch state, advanced by the kernel itself so a captured
@@ -1097,7 +1101,7 @@ extern "C" int plq_ensemble_create(plq_ctx *ctx, int32_t n, const plq_chain_desc
         a.seed32 = plq_fold_seed(d.seed);
         a.words = !(d.flags & PLQ_FLAG_GENERIC_PASS) &&
                   words_eligible(d.model, q, d.d, a.g.L, d.updater, d.rng) ? 1 : 0;
-        mem.wpt = tuned_wpt(d);
+        mem.wpt = tuned_wpt(d, packed_eligible(d));
         ModelParams p;
         std::memset(&p, 0, sizeof p);
         p.model = d.model;
@@ -1962,7 +1966,7 @@ int job_admit(ServerJob *j, cudaStream_t stream) {
     a.seed32 = plq_fold_seed(d.seed);
     a.words = !(d.flags & PLQ_FLAG_GENERIC_PASS) &&
               words_eligible(d.model, q, d.d, a.g.L, d.updater, d.rng) ? 1 : 0;
-    mem.wpt = tuned_wpt(d);
+    mem.wpt = tuned_wpt(d, packed_eligible(d));
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void **p, size_t bytes) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
