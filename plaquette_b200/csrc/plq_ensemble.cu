@@ -113,7 +113,7 @@ ShapeKey shape_key(const plq_chain_desc &d) {
 // Packed members start at one row a thread: a row is eight and more decisions,
 // and the tuner chose one for every shape of the workloads (256 tempered Ising
 // replicas of 16^3 to 64^3 beside 64 gauge lattices of 8^4 to 24^4: 148 us a sweep
-// at four, @@WPT at one).
+// at four, 119 at one).
 int tuned_wpt(const plq_chain_desc &d, bool packed) {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tuned.find(shape_key(d));
@@ -207,7 +207,7 @@ struct PackEntry {
 
 // Bytes to bits (unpack = false) or back (unpack = true) for every packed
 // member of the launch: one thread per row of one direction.
-__global__ void pack_links_kernel(const PackEntry *tab, int n_tab, uint32_t total, bool unpack) {
+__device__ void pack_rows(const PackEntry *tab, int n_tab, uint32_t total, bool unpack) {
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
         int lo = 0, hi = n_tab - 1;
         while (lo < hi) {  // the entry holding g
@@ -244,6 +244,10 @@ __global__ void pack_links_kernel(const PackEntry *tab, int n_tab, uint32_t tota
             }
         }
     }
+}
+
+__global__ void pack_links_kernel(const PackEntry *tab, int n_tab, uint32_t total, bool unpack) {
+    pack_rows(tab, n_tab, total, unpack);
 }
 
 // The pass-specific fields of member m's arguments for colour pass `sp` of
@@ -698,7 +702,7 @@ struct plq_ensemble {
     // work items for the current configuration
     int ranks = 4;
     int ctas_per_sm = 2;
-    bool words_only = false;  // every member runs four sites at a time
+    bool words_only = false;  // no member needs the generic body (runs_lean)
     WorkItem *d_items = nullptr;
     int64_t n_items = 0;
     int32_t *d_e_member = nullptr, *d_e_chunk = nullptr;
@@ -716,6 +720,7 @@ struct plq_ensemble {
     uint32_t pack_total = 0;
     // every member's primaries: one device buffer, the launches captured once
     long long *d_prims_all = nullptr;
+    uint8_t *d_links = nullptr;  // plq_ensemble_read's staging of link members
     std::vector<int64_t> prims_offset;  // member m's first entry
     PrimTask *d_prim_tasks = nullptr;   // every member's measurement task (the states never move)
     int32_t *d_prim_task = nullptr, *d_prim_chunk = nullptr;
@@ -771,7 +776,7 @@ int64_t item_cost(const EnsMember &mem, int64_t c, int ranks) {
     } else if (a.words) {
         unit_cost = 400;  // four sites of one colour in bytes
     } else {
-        unit_cost = 150;  // one colour rank, generic body
+        unit_cost = mem.link || a.jump ? 150 : 90;  // one colour rank, generic body or keyed site
     }
     return busiest * unit_cost;
 }
@@ -956,6 +961,10 @@ cudaError_t launch_ensemble(plq_ensemble *E, EnsArgs &a, const PackEntry *tab = 
     }
     return e;
 }
+
+// Members the kernel without the generic body takes: packed, four sites at a time,
+// or keyed sites one at a time.
+bool runs_lean(const EnsMember &m) { return m.pk || m.a.words || (!m.link && !m.a.jump); }
 
 cudaError_t launch_persistent(plq_ensemble *E, uint64_t sweeps) {
     EnsArgs a = ens_args(E, sweeps);
@@ -1226,7 +1235,7 @@ extern "C" int plq_ensemble_create(plq_ctx *ctx, int32_t n, const plq_chain_desc
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(E->stream);
     if (ce != cudaSuccess) return fail(ens_fail(ce, "ensemble set-up"));
     E->words_only = true;
-    for (auto &m : E->members) E->words_only = E->words_only && m.a.words;
+    for (auto &m : E->members) E->words_only = E->words_only && runs_lean(m);
     E->ctas_per_sm = std::max(1, std::min(4, max_ctas_per_sm(E->ranks, E->words_only)));
     int rc = build_items(E);
     if (rc != PLQ_OK) return fail(rc);
@@ -1700,12 +1709,16 @@ extern "C" int plq_ensemble_read(plq_ensemble *E, int32_t m, uint8_t *out) {
     const EnsMember &mem = E->members[m];
     cudaError_t e = cudaSuccess;
     if (mem.link) {
-        uint8_t *tmp = nullptr;
-        e = cudaMalloc((void **)&tmp, (size_t)mem.n_vars);
-        if (e == cudaSuccess) e = launch_planes_to_links(mem.a.state, tmp, mem.a.g.n_sites, mem.a.g.d, E->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(out, tmp, (size_t)mem.n_vars, cudaMemcpyDeviceToHost, E->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(E->stream);
-        if (tmp) cudaFree(tmp);
+        // host order through one staging buffer, as large as the largest link member, kept
+        if (!E->d_links) {
+            size_t most = 0;
+            for (const EnsMember &m2 : E->members)
+                if (m2.link) most = std::max(most, (size_t)m2.n_vars);
+            e = cudaMalloc((void **)&E->d_links, most);
+            if (e == cudaSuccess) E->allocs.push_back(E->d_links);
+        }
+        if (e == cudaSuccess) e = launch_planes_to_links(mem.a.state, E->d_links, mem.a.g.n_sites, mem.a.g.d, E->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(out, E->d_links, (size_t)mem.n_vars, cudaMemcpyDeviceToHost, E->stream);
     } else {
         e = cudaMemcpyAsync(out, mem.a.state, (size_t)mem.n_vars, cudaMemcpyDeviceToHost, E->stream);
     }
@@ -1934,8 +1947,28 @@ void job_release(ServerJob *j) {
     j->allocs.clear();
 }
 
+int64_t desc_vars(const plq_chain_desc &d) {
+    int64_t n = 1;
+    for (int i = 0; i < d.d; ++i) n *= d.shape[i];
+    return d.model == PLQ_GAUGE ? n * d.d : n;
+}
+
+// A packed job's rows from its bytes, or back.
+__global__ void pack_job_kernel(PackEntry entry, uint32_t total, bool unpack) { pack_rows(&entry, 1, total, unpack); }
+cudaError_t job_repack(const ServerJob *j, bool unpack, cudaStream_t stream) {
+    PackEntry t;
+    std::memset(&t, 0, sizeof t);
+    t.state = j->mem.a.state;
+    t.pk = j->mem.pk;
+    t.L0 = (uint32_t)j->mem.a.g.L[0];
+    t.wide = j->mem.pk_wide;
+    const uint32_t total = (uint32_t)(j->mem.n_vars / j->mem.a.g.L[0]);
+    pack_job_kernel<<<std::min<uint32_t>((total + 255) / 256, 148u * 8u), 256, 0, stream>>>(t, total, unpack);
+    return cudaGetLastError();
+}
+
 // Allocate and upload a job's resident state (worker thread, device current).
-int job_admit(ServerJob *j, cudaStream_t stream) {
+int job_admit(ServerJob *j, bool room_for_rows, cudaStream_t stream) {
     const plq_chain_desc &d = j->desc;
     EnsMember &mem = j->mem;
     std::memset(&mem, 0, sizeof mem);
@@ -1966,12 +1999,19 @@ int job_admit(ServerJob *j, cudaStream_t stream) {
     a.seed32 = plq_fold_seed(d.seed);
     a.words = !(d.flags & PLQ_FLAG_GENERIC_PASS) &&
               words_eligible(d.model, q, d.d, a.g.L, d.updater, d.rng) ? 1 : 0;
-    mem.wpt = tuned_wpt(d, packed_eligible(d));
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void **p, size_t bytes) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
         if (e == cudaSuccess) j->allocs.push_back(*p);
     };
+    // q = 2 and gauge jobs stay packed from admission to retirement, where the server's budget
+    // has room for the rows beside the bytes (a job is admitted on its bytes alone)
+    const bool packed = room_for_rows && packed_eligible(d);
+    mem.wpt = tuned_wpt(d, packed);
+    if (packed) {
+        alloc(&mem.pk, packed_bytes(d, mem.n_vars));
+        mem.pk_wide = d.model != PLQ_GAUGE && d.shape[0] > 32 ? 1 : 0;
+    }
     uint8_t *st = nullptr;
     alloc((void **)&st, (size_t)mem.n_vars);
     a.state = st;
@@ -1992,6 +2032,7 @@ int job_admit(ServerJob *j, cudaStream_t stream) {
             e = cudaMemsetAsync(st, 0, (size_t)mem.n_vars, stream);
         }
     }
+    if (e == cudaSuccess && mem.pk) e = job_repack(j, false, stream);
     if (e == cudaSuccess && d.rng == PLQ_RNG_STREAM) {
         uint64_t slo, shi, ilo, ihi;
         pcg_seed_from_u64(d.seed, slo, shi, ilo, ihi);
@@ -2066,14 +2107,14 @@ struct TickBuffers {
 
 int run_tick(plq_server *S, TickBuffers &B, cudaStream_t stream, uint64_t sweeps) {
     const size_t n = S->active.size();
-    // members that run four sites at a time first: they go to the words-only kernel
-    // (few registers, several CTAs per SM), the rest to a second launch of the full kernel
+    // members that need no generic body first: they go to the kernel without it (few registers,
+    // several CTAs per SM), the rest to a second launch of the full kernel
     std::vector<size_t> order;
     for (size_t m = 0; m < n; ++m)
-        if (S->active[m]->mem.a.words) order.push_back(m);
+        if (runs_lean(S->active[m]->mem)) order.push_back(m);
     const size_t nw = order.size();
     for (size_t m = 0; m < n; ++m)
-        if (!S->active[m]->mem.a.words) order.push_back(m);
+        if (!runs_lean(S->active[m]->mem)) order.push_back(m);
     std::vector<EnsMember> mems(n);
     std::vector<TableSet> tss(n);
     std::vector<int32_t> ts(n);
@@ -2185,7 +2226,8 @@ void retire(plq_server *S, ServerJob *j, cudaStream_t stream) {
     int np = primaries_count(mem.a.model, mem.a.q);
     std::vector<long long> prim((size_t)np, 0);
     long long *d = nullptr;
-    cudaError_t e = cudaMalloc((void **)&d, sizeof(long long) * (size_t)np);
+    cudaError_t e = mem.pk ? job_repack(j, true, stream) : cudaSuccess;
+    if (e == cudaSuccess) e = cudaMalloc((void **)&d, sizeof(long long) * (size_t)np);
     if (e == cudaSuccess) e = launch_primaries(mem.a.state, mem.a.g, mem.a.model, mem.a.q, d, stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(prim.data(), d, sizeof(long long) * (size_t)np, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess && j->want_states) {
@@ -2245,7 +2287,17 @@ void worker_loop(plq_server *S) {
             }
         }
         for (ServerJob *j : admit) {
-            int rc = job_admit(j, stream);
+            bool rows = false;
+            if (packed_eligible(j->desc)) {  // the packed rows, where the budget has room for them
+                const uint64_t bytes = packed_bytes(j->desc, desc_vars(j->desc));
+                std::lock_guard<std::mutex> lock(S->mu);
+                rows = S->used + bytes <= S->budget;
+                if (rows) {
+                    S->used += bytes;
+                    j->footprint += bytes;
+                }
+            }
+            int rc = job_admit(j, rows, stream);
             std::lock_guard<std::mutex> lock(S->mu);
             if (rc != PLQ_OK) {
                 S->used -= j->footprint;

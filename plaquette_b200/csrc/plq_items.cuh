@@ -32,16 +32,93 @@ __device__ void run_words(const LocalArgs &a, int link, int64_t chunk, int R) {
     }
 }
 
-// WORDS_ONLY: every member runs four sites at a time, so the generic body is
-// compiled out (far fewer registers, more CTAs per SM).
+// Keyed sites in bytes, one colour site at a time: any q, any even extents (the
+// lattices whose rows the four-site words do not fit, and every Potts Metropolis
+// chain).  The same keys, draws and tables as plq_local_impl.cuh; that body's
+// eight ranks a thread, 64-bit keys and unused packing weights left the pass at two
+// CTAs per SM: q = 5 Metropolis on 1002 x 750, 20.6 us a sweep, 10.1 so.
+template <int D>
+__device__ __forceinline__ void rank_site(const LocalArgs &p, uint32_t r, uint32_t mix) {
+    const uint32_t q = (uint32_t)p.q;
+    const bool metropolis = p.kernel == PLQ_METROPOLIS;
+    int32_t x[D], op[D], om[D];
+    const uint32_t s = site_of_rank<D>(p.g, r, p.color, x);
+    wrap_offsets<D>(p.g, x, op, om);
+    const uint32_t cur = p.state[s];
+    uint32_t nb[2 * D];
+#pragma unroll
+    for (int mu = 0; mu < D; ++mu) {
+        nb[2 * mu] = p.state[s + (uint32_t)op[mu]];
+        nb[2 * mu + 1] = p.state[s + (uint32_t)om[mu]];
+    }
+    const uint32_t k = lowbias32_tail(lowbias32_head(p.seed32 ^ s) ^ mix) >> 8;
+    uint32_t out = cur;
+    if (metropolis && q > 2) {
+        // keyed proposal (metropolis.wgsl:45-55)
+        const uint32_t k24 = lowbias32_tail(lowbias32_head(p.seed32 ^ kProposalKey ^ s) ^ mix) >> 8;
+        const float scaled = __fmul_rn(__fmul_rn((float)k24, 5.9604644775390625e-8f), (float)(q - 1));
+        uint32_t prop = __float2uint_rz(scaled);
+        if (prop >= q - 1) prop = q - 2;
+        if (prop >= cur) prop += 1;
+        uint32_t cp = 0, cc = 0;
+#pragma unroll
+        for (int i = 0; i < 2 * D; ++i) {
+            cp += nb[i] == prop;
+            cc += nb[i] == cur;
+        }
+        constexpr uint32_t B = 2 * D + 1;
+        const uint32_t e = p.metro24[((cur * q + prop) * B + cp) * B + cc];
+        if (e == 0xFFFFFFFFu || k < e) out = prop;
+    } else {
+        uint32_t key = 0;
+#pragma unroll
+        for (int i = 0; i < 2 * D; ++i) key += (uint32_t)p.pw[nb[i]];
+        key = cur + q * key;
+        if (metropolis) {
+            const uint32_t e = p.metro24[key];
+            if (e == 0xFFFFFFFFu || k < e) out = 1u - cur;
+        } else {
+            const uint32_t *cut = p.hb24 + (size_t)key * (q - 1);
+            out = 0;
+            for (uint32_t j = 0; j + 1 < q; ++j) out += cut[j] <= k ? 1u : 0u;
+        }
+    }
+    p.state[s] = (uint8_t)out;
+}
+
+// One chunk of a colour pass: blockDim.x * R ranks, a thread's blockDim.x apart.
+template <int D, int R>
+__device__ __forceinline__ void rank_chunk(const LocalArgs &a, int64_t chunk) {
+    const uint32_t half = (uint32_t)(a.g.n_sites / 2), mix = keyed_mix(a.sweep32);
+    const uint32_t r0 = (uint32_t)(chunk * (int64_t)blockDim.x * R) + threadIdx.x;
+#pragma unroll 1
+    for (int i = 0; i < R; ++i) {
+        const uint32_t r = r0 + (uint32_t)i * blockDim.x;
+        if (r < half) rank_site<D>(a, r, mix);
+    }
+}
+
+// WORDS_ONLY: every member runs four sites at a time, packed, or as keyed sites one
+// at a time, so the generic body is compiled out (far fewer registers, more CTAs
+// per SM).
 template <int R, bool WORDS_ONLY>
 __device__ void run_item(const LocalArgs &a, int d, int link, int64_t chunk, int wpt) {
-    if (WORDS_ONLY || a.words) {
+    if (a.words) {
         switch (d) {
             case 1: run_words<1>(a, link, chunk, wpt); break;
             case 2: run_words<2>(a, link, chunk, wpt); break;
             case 3: run_words<3>(a, link, chunk, wpt); break;
             case 4: run_words<4>(a, link, chunk, wpt); break;
+            default: break;
+        }
+        return;
+    }
+    if (!link && !a.jump) {
+        switch (d) {
+            case 1: rank_chunk<1, R>(a, chunk); break;
+            case 2: rank_chunk<2, R>(a, chunk); break;
+            case 3: rank_chunk<3, R>(a, chunk); break;
+            case 4: rank_chunk<4, R>(a, chunk); break;
             default: break;
         }
         return;
