@@ -22,6 +22,7 @@
 #include "plq_device.cuh"
 #include "plq_fused.h"
 #include "plq_local.h"
+#include "plq_readback.h"
 #include "plq_measure.h"
 #include "plq_scan.h"
 #include "plq_tables.h"
@@ -839,9 +840,9 @@ extern "C" int plq_chain_read(plq_chain *c, uint8_t *out) {
         int rc = ensure_io(c);
         if (rc == PLQ_OK) rc = state_to_host_order(c, c->d_io);
         if (rc != PLQ_OK) return rc;
-        PLQ_CUDA(cudaMemcpyAsync(out, c->d_io, (size_t)c->n_vars, cudaMemcpyDeviceToHost, c->stream), "read");
+        PLQ_CUDA(plq_readback(out, c->d_io, (size_t)c->n_vars, c->ctx->device, c->stream), "read");
     } else {
-        PLQ_CUDA(cudaMemcpyAsync(out, c->d_state, (size_t)c->n_vars, cudaMemcpyDeviceToHost, c->stream), "read");
+        PLQ_CUDA(plq_readback(out, c->d_state, (size_t)c->n_vars, c->ctx->device, c->stream), "read");
     }
     return check_status(c);
 }
@@ -1052,8 +1053,7 @@ extern "C" int plq_chain_next_batch(plq_chain *c, int64_t count, uint8_t *out_st
                 c->measuring[k] = false;
             }
         if (out_states)
-            PLQ_CUDA(cudaMemcpyAsync(out_states + done * c->n_vars, c->d_snap, (size_t)(m * c->n_vars),
-                                     cudaMemcpyDeviceToHost, c->stream),
+            PLQ_CUDA(plq_readback(out_states + done * c->n_vars, c->d_snap, (size_t)(m * c->n_vars), c->ctx->device, c->stream),
                      "batch read-back");
         if (out_primaries)
             PLQ_CUDA(cudaMemcpyAsync(out_primaries + done * np, c->d_snap_obs, sizeof(long long) * (size_t)(m * np),

@@ -50,6 +50,7 @@
 #include "plq_device.cuh"
 #include "plq_geom.cuh"
 #include "plq_local.h"
+#include "plq_readback.h"
 #include "plq_tables.h"
 
 using namespace plq;
@@ -1725,8 +1726,7 @@ int cluster_labels(plq_chain *c, int32_t *out) {
     ClusterDev *cd = static_cast<ClusterDev *>(c->cl);
     if (!cd || !cd->decomposed) return plq_fail(PLQ_EINVAL, "no decomposition yet (run a Swendsen-Wang sweep first)");
     flatten(c);
-    cudaError_t e = cudaMemcpyAsync(out, cd->parent, sizeof(int32_t) * (size_t)c->n_sites, cudaMemcpyDeviceToHost,
-                                    c->stream);
+    cudaError_t e = plq_readback(out, cd->parent, sizeof(int32_t) * (size_t)c->n_sites, c->ctx->device, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return plq_fail(PLQ_ECUDA, std::string("labels read: ") + cudaGetErrorString(e));
     return PLQ_OK;
