@@ -26,16 +26,15 @@
 //               forced-change proposal) at consecutive positions, inside the
 //               rank scan; rand's range sampler occasionally takes a second
 //               draw, which shifts every later cluster -- those rare events
-//               are reported by the scan and fixed up by re-running the
-//               (parallel) draw pass with the events known, in a short host
-//               loop.
+//               are reported by the scan and fixed up by drawing the labels
+//               again with the events known (settle_labels_kernel).
 //
 // Wolff on the keyed stream: the reference relabels the cluster of a keyed
 // seed site in the full decomposition (cluster_relabel.wgsl:55-66).  Here one
 // persistent launch runs all requested updates: a CTA grows the cluster from
 // the seed site for a few generations while the others label the tiles
-// (wolff_kernel); its minimum site is the root the forced change is keyed on.  Wolff on the PCG stream (draws in grow_cluster's FIFO order)
-// is sequential by definition and is not run on the device.
+// (wolff_kernel); its minimum site is the root the forced change is keyed on.
+// Wolff on the PCG stream (draws in grow_cluster's FIFO order) is sequential by definition and is not run on the device.
 //
 // Every loop that waits or retries has an iteration cap; hitting one sets a
 // status bit the host turns into PLQ_ECAP / PLQ_EDEVICE.
@@ -62,6 +61,7 @@ constexpr int kSitesPerThread = 8;
 constexpr int kChunk = kThreads * kSitesPerThread;
 constexpr int kSpinLimit = 1 << 22;
 constexpr int kMaxEvents = 64;
+constexpr int kNoEvent = 0x7FFFFFFF;
 constexpr unsigned long long kDescAgg = 1ull, kDescPrefix = 2ull;
 
 struct ClusterArgs {
@@ -82,16 +82,16 @@ struct ClusterArgs {
     uint32_t kp24;   // keyed: bond open iff k24 < kp24
     uint64_t kp53;   // stream: bond open iff k53 < kp53
     const Affine *jump;
-    u128 base, inc;
+    u128 inc;
+    u128 *at;        // stream states: of the draw at ctrl->pos[0] (the sweep's first), and at pos[1] (its first label)
     Control *ctrl;
     unsigned long long *desc;
     int64_t n_chunks;
     uint64_t ticket_base;
     uint32_t epoch;
     int cap;          // iteration cap of finds and unions
-    const int32_t *events;  // sorted ranks of clusters that take two draws
-    int n_events;
-    int *first_new;   // device: smallest rank with an unknown second draw
+    int32_t *events;  // device: sorted ranks of clusters that take two draws
+    int *first_new;   // device: smallest rank with an unknown second draw; [1]: the number of events
     uint64_t updates; // Wolff: updates in this launch
 };
 
@@ -257,24 +257,31 @@ __global__ void __launch_bounds__(kThreads) bonds_kernel(ClusterArgs a) {
             count += __popc(m);
         }
     }
-    u128 st{0, 0};
+    u128 st{0, 0}, chunk_state{0, 0};
+    uint64_t chunk_draws = 0;
     if (STREAM) {
         int total;
         bool ok;
         uint64_t excl = chunk_scan(a, chunk, count, total, ok);
         if (!ok) return;
+        chunk_draws = (uint64_t)total;
         // One full jump per chunk, to its first draw (thread 0's prefix is the chunk's); each
         // thread then applies the low digits of its offset inside the chunk (< kChunk * D draws).
         // Jump maps are iterates of one affine map, so they compose in any order.
         __shared__ unsigned long long s_base, s_excl0;
         __shared__ u128 s_state;
         if (threadIdx.x == 0) {
+            if (chunk == 0) {  // this sweep's second draws: none known
+                a.first_new[0] = kNoEvent;
+                a.first_new[1] = 0;
+            }
             s_base = a.ctrl->pos[0];
             if (chunk == a.n_chunks - 1) a.ctrl->pos[1] = s_base + excl + (unsigned long long)total;
             s_excl0 = excl;
-            s_state = jump(a.jump, a.base, s_base + excl);
+            s_state = jump(a.jump, a.at[0], excl);
         }
         __syncthreads();
+        chunk_state = s_state;
         if (count) st = jump(a.jump, s_state, excl - s_excl0);
     }
     uint64_t opened = 0;
@@ -300,6 +307,7 @@ __global__ void __launch_bounds__(kThreads) bonds_kernel(ClusterArgs a) {
         else a.bonds[s] = open;
     }
     if (row8 && s0 < n) *reinterpret_cast<uint64_t *>(a.bonds + s0) = opened;
+    if (STREAM && chunk == a.n_chunks - 1 && threadIdx.x == 0) a.at[1] = jump(a.jump, chunk_state, chunk_draws);
 }
 
 // ------------------------------------------------------------ 2. labels
@@ -953,8 +961,8 @@ __device__ __forceinline__ uint32_t fresh_label(const ClusterArgs &a, u128 st, u
 // stream: rank of each root among roots (first-encounter order), and each
 // root's fresh label drawn with no second draws known: rank r draws at
 // bond_end + r, so a thread steps the stream from one root to the next.  A root
-// whose label takes a second draw reports its rank in first_new; the host then
-// re-runs the draws (root_draw_kernel) with that event known.
+// whose label takes a second draw reports its rank in first_new; settle_labels_kernel
+// then draws the labels again with that event known.
 template <int D>
 __global__ void __launch_bounds__(kThreads) root_rank_kernel(ClusterArgs a) {
     const int64_t n = a.g.n_sites;
@@ -989,13 +997,15 @@ __global__ void __launch_bounds__(kThreads) root_rank_kernel(ClusterArgs a) {
     if (threadIdx.x == 0) {
         if (chunk == a.n_chunks - 1) a.ctrl->scratch[0] = excl + (unsigned long long)total;
         // labels are drawn from the end of the bond draws, in root rank order
-        const u128 st0 = jump(a.jump, a.base, a.ctrl->pos[1] + excl);
+        const u128 st0 = jump(a.jump, a.at[1], excl);
         a.chunk_base[chunk].st = st0;
         a.chunk_base[chunk].rank0 = (int64_t)excl;
         s_state = st0;
         s_excl0 = excl;
     }
     __syncthreads();
+    // the state after the labels (settle_labels_kernel adds second draws), beside the draws
+    if (chunk == a.n_chunks - 1 && threadIdx.x == kThreads - 1) a.at[0] = jump(a.jump, s_state, (uint64_t)total);
     if (!count) return;
     u128 st = jump(a.jump, s_state, excl - s_excl0);
     int r = (int)excl;
@@ -1012,31 +1022,68 @@ __global__ void __launch_bounds__(kThreads) root_rank_kernel(ClusterArgs a) {
     }
 }
 
-// stream: each root draws its cluster's fresh label (ClusterUpdate::fresh_label,
-// updater.rs:507-521) at bond_end + rank + (known second draws before it),
-// jumping from its root_rank chunk's first label draw.
+// stream, after the rank pass: where a label took a second draw, every label again
+// -- each root draws its cluster's fresh label (ClusterUpdate::fresh_label,
+// updater.rs:507-521) at bond_end + rank + (known second draws before it), jumping
+// from its root_rank chunk's first label draw -- until no unknown second draw
+// turns up; then the stream position after the sweep.  One CTA: such a draw comes
+// once in 2^32 / (q - 1) labels, and a launch that finds none costs less than
+// asking the host (3D Potts q = 3 96^3: 91 us a sweep with the host's answer,
+// 72 so).
+constexpr int kSettleThreads = 256;
 template <int D, bool SMALL>
-__global__ void __launch_bounds__(kThreads) root_draw_kernel(ClusterArgs a) {
+__global__ void __launch_bounds__(kSettleThreads) settle_labels_kernel(ClusterArgs a, uint32_t n_tiles) {
     using T = Tile<D, SMALL>;
-    const T t(a.g);
-    int xt[3];
-    const uint32_t s_tile = t.origin(blockIdx.x, xt);
-    for (uint32_t li = threadIdx.x; li < T::kSites; li += kThreads) {
-        if (!t.inside(xt, li) || a.local_root[(size_t)blockIdx.x * T::kSites + li] != li) continue;
-        const int64_t s = t.site(s_tile, li);
-        if (a.parent[s] != (int32_t)s) continue;
-        int32_t r = a.rank[s];
-        int before = 0;
-        bool known = false;
-        for (int e = 0; e < a.n_events; ++e) {
-            before += a.events[e] < r;
-            known |= a.events[e] == r;
+    __shared__ int s_n;
+    volatile int *first_new = a.first_new;
+    for (int n = 0;; ++n) {
+        __syncthreads();
+        const int first = first_new[0];
+        __syncthreads();  // (all have read it)
+        if (first == kNoEvent) {
+            if (threadIdx.x == 0) {
+                a.ctrl->pos[0] = a.ctrl->pos[1] + a.ctrl->scratch[0] + (unsigned long long)n;
+                for (int k = 0; k < n; ++k) a.at[0] = pcg_step(a.at[0], a.inc);
+            }
+            return;
         }
-        const ClusterArgs::ChunkBase &cb = a.chunk_base[s / kChunk];
-        const u128 st = jump(a.jump, cb.st, (uint64_t)((int64_t)r - cb.rank0) + (uint64_t)before);
-        bool second;
-        a.fresh[s] = (uint8_t)fresh_label(a, st, a.state[s], second);
-        if (second && !known) atomicMin(a.first_new, r);
+        if (n == kMaxEvents) {
+            if (threadIdx.x == 0) atomicOr(&a.ctrl->status, kStatusQueueOverflow);
+            return;
+        }
+        if (threadIdx.x == 0) {  // into the sorted list
+            int k = n;
+            for (; k > 0 && a.events[k - 1] > first; --k) a.events[k] = a.events[k - 1];
+            a.events[k] = first;
+            s_n = n + 1;
+            first_new[0] = kNoEvent;
+            __threadfence();
+        }
+        __syncthreads();
+        const int known_n = s_n;
+        const T t(a.g);
+        for (uint32_t tile = 0; tile < n_tiles; ++tile) {
+            int xt[3];
+            const uint32_t s_tile = t.origin(tile, xt);
+            for (uint32_t li = threadIdx.x; li < T::kSites; li += kSettleThreads) {
+                if (!t.inside(xt, li) || a.local_root[(size_t)tile * T::kSites + li] != li) continue;
+                const int64_t s = t.site(s_tile, li);
+                if (a.parent[s] != (int32_t)s) continue;
+                const int32_t r = a.rank[s];
+                int before = 0;
+                bool known = false;
+                for (int e = 0; e < known_n; ++e) {
+                    before += a.events[e] < r;
+                    known |= a.events[e] == r;
+                }
+                const ClusterArgs::ChunkBase &cb = a.chunk_base[s / kChunk];
+                const u128 st = jump(a.jump, cb.st, (uint64_t)((int64_t)r - cb.rank0) + (uint64_t)before);
+                bool second;
+                a.fresh[s] = (uint8_t)fresh_label(a, st, a.state[s], second);
+                if (second && !known) atomicMin(a.first_new, r);
+            }
+        }
+        __threadfence();
     }
 }
 
@@ -1050,10 +1097,6 @@ __global__ void __launch_bounds__(kThreads) apply_fresh_kernel(ClusterArgs a) {
             const uint8_t v[4] = {value[r[0]], value[r[1]], value[r[2]], value[r[3]]};
             store_row(a.state, s, count, v);
         });
-}
-
-__global__ void finish_pos_kernel(Control *ctrl, int n_events) {
-    ctrl->pos[0] = ctrl->pos[1] + ctrl->scratch[0] + (unsigned long long)n_events;
 }
 
 // ------------------------------------------------------- Wolff (keyed)
@@ -1392,7 +1435,7 @@ struct ClusterDev {
     uint32_t kp24 = 0;
     uint64_t kp53 = 0;
     uint64_t lookback_launches = 0;
-    std::vector<int32_t> host_events;
+    u128 *at = nullptr;
     bool decomposed = false;
     bool flat = false;  // every site's parent is its root (flatten_kernel has run since the last sweep)
 };
@@ -1423,7 +1466,7 @@ ClusterArgs cluster_args(plq_chain *c) {
     a.kp24 = cd->kp24;
     a.kp53 = cd->kp53;
     a.jump = c->d_jump;
-    a.base = c->base;
+    a.at = cd->at;
     a.inc = c->inc;
     a.ctrl = c->d_ctrl;
     a.desc = cd->desc;
@@ -1432,14 +1475,6 @@ ClusterArgs cluster_args(plq_chain *c) {
     a.events = cd->events;
     a.first_new = cd->first_new;
     return a;
-}
-
-// The range of the per-cluster label draw: next_below(q) to redraw
-// (src/updater.rs:512), propose's next_below(q - 1) for the forced change
-// (:515, :659-668; a range of 1 at q = 2, which consumes nothing).
-bool label_range_is_power_of_two(const plq_chain *c) {
-    const uint32_t range = c->desc.relabel == PLQ_RELABEL_FORCED ? (uint32_t)c->q - 1u : (uint32_t)c->q;
-    return (range & (range - 1u)) == 0u;
 }
 
 // The kernels of one tile size (a CTA per tile, and the boundary unions).
@@ -1457,8 +1492,8 @@ struct TileKernels {
     static void relabel_keyed(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
         relabel_keyed_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
     }
-    static void root_draw(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
-        root_draw_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
+    static void settle(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
+        settle_labels_kernel<D, SMALL><<<1, kSettleThreads, 0, st>>>(a, tiles);
     }
     static void apply_fresh(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
         apply_fresh_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
@@ -1521,45 +1556,13 @@ int sweep_t(plq_chain *c, uint64_t sweeps) {
         if (!stream) {
             K::relabel_keyed(a, (unsigned)cd->n_tiles, c->stream);
             c->launches++;
-        } else if (label_range_is_power_of_two(c)) {
-            // rand's range sampler never takes a second draw for a power-of-two range
-            // (x * 2^k leaves its low word a multiple of 2^k, never inside the rejection
-            // zone above 2^32 - 2^k): the labels drawn by the rank pass are final and the
-            // sweep needs no round-trip to the host
-            lookback(a);
-            root_rank_kernel<D><<<(unsigned)cd->n_chunks, kThreads, 0, c->stream>>>(a);
-            K::apply_fresh(a, (unsigned)cd->n_tiles, c->stream);
-            finish_pos_kernel<<<1, 1, 0, c->stream>>>(c->d_ctrl, 0);
-            c->launches += 3;
         } else {
             lookback(a);
-            const int none = 0x7FFFFFFF;
-            cudaMemcpyAsync(cd->first_new, &none, sizeof none, cudaMemcpyHostToDevice, c->stream);
-            // ranks, and the labels with no second draws known
+            // ranks, and the labels with no second draws known; the second draws; the labels to the sites
             root_rank_kernel<D><<<(unsigned)cd->n_chunks, kThreads, 0, c->stream>>>(a);
-            c->launches++;
-            cd->host_events.clear();
-            for (int round = 0;; ++round) {
-                if (round > 0) {  // again, with the second draws found so far known
-                    a.n_events = (int)cd->host_events.size();
-                    cudaMemcpyAsync(cd->first_new, &none, sizeof none, cudaMemcpyHostToDevice, c->stream);
-                    cudaMemcpyAsync(cd->events, cd->host_events.data(), sizeof(int32_t) * a.n_events,
-                                    cudaMemcpyHostToDevice, c->stream);
-                    K::root_draw(a, (unsigned)cd->n_tiles, c->stream);
-                    c->launches++;
-                }
-                int first = none;
-                cudaMemcpyAsync(&first, cd->first_new, sizeof first, cudaMemcpyDeviceToHost, c->stream);
-                cudaError_t e = cudaStreamSynchronize(c->stream);
-                if (e != cudaSuccess) return plq_fail(PLQ_ECUDA, std::string("root draws: ") + cudaGetErrorString(e));
-                if (first == none) break;
-                if ((int)cd->host_events.size() >= kMaxEvents)
-                    return plq_fail(PLQ_EDEVICE, "too many two-draw label events in one sweep");
-                cd->host_events.insert(std::upper_bound(cd->host_events.begin(), cd->host_events.end(), first), first);
-            }
+            K::settle(a, (unsigned)cd->n_tiles, c->stream);
             K::apply_fresh(a, (unsigned)cd->n_tiles, c->stream);
-            finish_pos_kernel<<<1, 1, 0, c->stream>>>(c->d_ctrl, (int)cd->host_events.size());
-            c->launches += 2;
+            c->launches += 3;
         }
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return plq_fail(PLQ_ECUDA, std::string("cluster sweep: ") + cudaGetErrorString(e));
@@ -1662,7 +1665,9 @@ int cluster_create(plq_chain *c) {
             alloc((void **)&cd->rank, sizeof(int32_t) * (size_t)n);
             alloc((void **)&cd->chunk_base, sizeof(ClusterArgs::ChunkBase) * (size_t)cd->n_chunks);
             alloc((void **)&cd->events, sizeof(int32_t) * kMaxEvents);
-            alloc((void **)&cd->first_new, sizeof(int));
+            alloc((void **)&cd->first_new, 2 * sizeof(int));
+            alloc((void **)&cd->at, 2 * sizeof(u128));
+            if (e == cudaSuccess) e = cudaMemcpyAsync(cd->at, &c->base, sizeof(u128), cudaMemcpyHostToDevice, c->stream);
         }
     }
     if (e != cudaSuccess)
@@ -1690,7 +1695,7 @@ int cluster_sweep(plq_chain *c) { return cluster_sweep_n(c, 1); }
 void cluster_free(plq_chain *c) {
     ClusterDev *cd = static_cast<ClusterDev *>(c->cl);
     if (!cd) return;
-    void *ptrs[] = {cd->bonds, cd->parent, cd->local_root, cd->fresh, cd->rank, cd->chunk_base, cd->wolff,
+    void *ptrs[] = {cd->bonds, cd->parent, cd->local_root, cd->fresh, cd->rank, cd->chunk_base, cd->wolff, cd->at,
                     cd->desc, cd->events, cd->first_new, cd->sizes};
     for (void *p : ptrs)
         if (p) cudaFree(p);
