@@ -1106,10 +1106,9 @@ __global__ void __launch_bounds__(kThreads) apply_fresh_kernel(ClusterArgs a) {
 // lattice does on all SMs (2D Ising 1024^2: 3.9 ms an update against 0.034).
 // But far from criticality, and for many seeds at it, the cluster is a few
 // sites, which a few generations find.  So one CTA of a persistent launch grows
-// each update's cluster and goes on to the next as long as they are small; at
-// generation kAnnounce it calls the others, which label the tiles as in a
-// Swendsen-Wang sweep while it grows on to kGrowGenerations (they stop when the
-// growth has ended first).  A cluster that outgrew the limits is the one the
+// each update's cluster and goes on to the next as long as they are small; half-way
+// to its limit it calls the others, which label the tiles as in a Swendsen-Wang
+// sweep while it grows on (they stop when the growth has ended first).  A cluster that outgrew the limits is the one the
 // seed site has in the decomposition.  Grid barriers: none for an update of
 // fewer generations, one where the growth ended after the call, three for a
 // large cluster.
@@ -1119,10 +1118,14 @@ __global__ void __launch_bounds__(kThreads) apply_fresh_kernel(ClusterArgs a) {
 // 592 / 26, 32 x 26 87 / 23, 3D Potts q = 3 80^3 60 / 19; 3D Ising 128^3 at
 // beta = 0.1 4.1 / 3.0.  Calling at generation 4 was 2 us faster on the smallest
 // lattices and 1.5 us slower on the hot one.
-constexpr int kAnnounce = 6;
-constexpr int kGrowGenerations = 12;
-constexpr uint32_t kGrowMembers = 1024;
-constexpr uint32_t kGrowTable = 4096;  // members' hash table: never more than half full
+//
+// The limits grow with the labelling they save: 12 generations, and one more for
+// each 32 tiles up to 28; the call comes half-way (3D Potts q = 4 128^3 in its
+// disordered phase, clusters of some 10^3 sites: 18 us an update by growth alone,
+// 25 with 12 generations everywhere, 11 so).
+__host__ __device__ inline int grow_generations(uint32_t n_tiles) { return 12 + (int)(n_tiles < 512u ? n_tiles / 32u : 16u); }
+constexpr uint32_t kGrowMembers = 2048;
+constexpr uint32_t kGrowTable = 8192;  // members' hash table: never more than half full
 static_assert(kGrowMembers + kThreads <= kGrowTable / 2, "room for a pass past the limit");
 
 struct GrowShared {
@@ -1191,10 +1194,10 @@ __device__ __forceinline__ void wolff_call(WolffSync *w, unsigned long long id) 
 // other CTAs were called to this update.
 template <int D>
 __device__ bool wolff_grow(const ClusterArgs &a, uint32_t sweep, uint32_t seed, uint8_t cur, GrowShared &sm, WolffSync *w,
-                           unsigned long long id, bool &called) {
+                           unsigned long long id, int generations, bool &called) {
     const BondCut cut(a, sweep);
     const bool bonds = BondCut::some(a);
-    auto slot_of = [](uint32_t v) { return (v * 0x9e3779b1u) >> 20; };  // kGrowTable = 2^12
+    auto slot_of = [](uint32_t v) { return (v * 0x9e3779b1u) >> 19; };  // kGrowTable = 2^13
     for (uint32_t i = threadIdx.x; i < kGrowTable; i += kThreads) sm.table[i] = -1;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1206,8 +1209,8 @@ __device__ bool wolff_grow(const ClusterArgs &a, uint32_t sweep, uint32_t seed, 
     __syncthreads();
     uint32_t begin = 0, end = 1;
     called = false;
-    for (int gen = 0; begin < end && gen < kGrowGenerations && end <= kGrowMembers; ++gen) {
-        if (gen == kAnnounce) {
+    for (int gen = 0; begin < end && gen < generations && end <= kGrowMembers; ++gen) {
+        if (gen == generations / 2) {
             wolff_call(w, id);
             called = true;
         }
@@ -1303,7 +1306,7 @@ wolff_kernel(ClusterArgs a, WolffSync *w, uint32_t n_tiles, unsigned long long l
             GrowShared &sm = *reinterpret_cast<GrowShared *>(s_buf);
             if (threadIdx.x == 0) a.ctrl->scratch[1] = 0;
             bool called;
-            const bool whole = wolff_grow<D>(a, sweep, seed, cur, sm, w, id, called);
+            const bool whole = wolff_grow<D>(a, sweep, seed, cur, sm, w, id, grow_generations(n_tiles), called);
             if (whole) {
                 // (the others may be reading states for tiles that no one will use)
                 const uint8_t next = wolff_next(a, sweep, sm.min_site, cur);
