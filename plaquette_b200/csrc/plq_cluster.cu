@@ -1108,8 +1108,8 @@ __global__ void __launch_bounds__(kThreads) apply_fresh_kernel(ClusterArgs a) {
 // sites, which a few generations find.  So one CTA of a persistent launch grows
 // each update's cluster and goes on to the next as long as they are small; half-way
 // to its limit it calls the others, which label the tiles as in a Swendsen-Wang
-// sweep while it grows on (they stop when the growth has ended first).  A cluster that outgrew the limits is the one the
-// seed site has in the decomposition.  Grid barriers: none for an update of
+// sweep while it grows on (they stop when the growth has ended first).  A cluster
+// that outgrew the limits is the one the seed site has in the decomposition.  Grid barriers: none for an update of
 // fewer generations, one where the growth ended after the call, three for a
 // large cluster.
 //
