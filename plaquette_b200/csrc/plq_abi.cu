@@ -505,6 +505,13 @@ extern "C" int plq_chain_create(plq_ctx *ctx, const plq_chain_desc *desc, const 
                 c->resident_totals = (plan.packed_bytes + 15) & ~(size_t)15;
                 if (plan.packed_bytes)
                     e = cudaMalloc(&c->d_resident, c->resident_totals + (plan.stream_draws ? kResidentTotals * sizeof(uint32_t) : 0));
+                if (e == cudaErrorMemoryAllocation) {  // a device too full for the words: the per-pass kernels
+                    c->d_resident = nullptr;
+                    c->resident = ResidentPlan();
+                    c->resident_totals = 0;
+                    cudaGetLastError();
+                    e = cudaSuccess;
+                }
                 if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc(resident words)"));
             }
         }
@@ -884,8 +891,12 @@ extern "C" int plq_chain_axis_pair_sums(plq_chain *c, int64_t *out, int64_t capa
     if (n_pairs) {
         cudaError_t e;
         const size_t words = pair_words_bytes(c->g, c->q);
-        if (words) {
-            if (!c->d_pair_words) PLQ_CUDA(cudaMalloc((void **)&c->d_pair_words, words), "cudaMalloc(pair words)");
+        // a device too full for the planes counts on the bytes
+        if (words && !c->d_pair_words && cudaMalloc((void **)&c->d_pair_words, words) != cudaSuccess) {
+            c->d_pair_words = nullptr;
+            cudaGetLastError();
+        }
+        if (words && c->d_pair_words) {
             e = launch_pair_bits(c->d_state, c->g, c->q, c->d_pair_words, n_pairs, c->d_meas, c->ctx->sm_count, c->stream);
         } else {
             PLQ_CUDA(cudaMemcpyAsync(c->d_pairs, pairs.data(), sizeof(int32_t) * 2 * (size_t)n_pairs,
