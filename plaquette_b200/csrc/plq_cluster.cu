@@ -51,6 +51,7 @@
 #include "plq_local.h"
 #include "plq_readback.h"
 #include "plq_tables.h"
+#include "plq_wolff_sync.h"
 
 using namespace plq;
 
@@ -1138,7 +1139,7 @@ struct GrowShared {
 struct WolffSync {
     unsigned int count, gen;      // the grid barrier's arrivals and generation
     unsigned long long call;      // the update the CTAs are called to label (increasing over all launches)
-    unsigned long long small[2];  // by update parity: the called update whose cluster the growth found whole
+    unsigned long long small[2];  // by update parity: the last called update whose cluster the growth found whole
 };
 
 // Grid barrier (all CTAs are co-resident: a cooperative launch); bounded.
@@ -1321,7 +1322,7 @@ wolff_kernel(ClusterArgs a, WolffSync *w, uint32_t n_tiles, unsigned long long l
         } else {
             LabelShared<T> &sm = *reinterpret_cast<LabelShared<T> *>(s_buf);
             for (uint32_t tile = blockIdx.x - 1u; tile < n_tiles; tile += gridDim.x - 1u) {
-                if (threadIdx.x == 0) s_stop = *small == id;
+                if (threadIdx.x == 0) s_stop = wolff_ended_by_growth(*small, id);
                 __syncthreads();
                 if (s_stop) break;
                 label_tile<D, SMALL, true>(a, sweep, tile, sm);
@@ -1329,7 +1330,7 @@ wolff_kernel(ClusterArgs a, WolffSync *w, uint32_t n_tiles, unsigned long long l
             }
         }
         wolff_barrier(w, a.ctrl);
-        if (threadIdx.x == 0) s_stop = *small == id;
+        if (threadIdx.x == 0) s_stop = wolff_ended_by_growth(*small, id);
         __syncthreads();
         if (s_stop) continue;
         unite_edges<D, SMALL, true>(a, sweep);
