@@ -720,7 +720,8 @@ struct plq_ensemble {
     uint32_t pack_total = 0;
     // every member's primaries: one device buffer, the launches captured once
     long long *d_prims_all = nullptr;
-    uint8_t *d_links = nullptr;  // plq_ensemble_read's staging of link members
+    uint8_t *d_links = nullptr;  // plq_ensemble_read's staging of link members,
+    std::mutex links_mu;         // one call's at a time (members may be read from several threads)
     std::vector<int64_t> prims_offset;  // member m's first entry
     PrimTask *d_prim_tasks = nullptr;   // every member's measurement task (the states never move)
     int32_t *d_prim_task = nullptr, *d_prim_chunk = nullptr;
@@ -1709,16 +1710,26 @@ extern "C" int plq_ensemble_read(plq_ensemble *E, int32_t m, uint8_t *out) {
     const EnsMember &mem = E->members[m];
     cudaError_t e = cudaSuccess;
     if (mem.link) {
-        // host order through one staging buffer, as large as the largest link member, kept
+        // host order through one staging buffer, as large as the largest link member, kept and used by
+        // one call at a time; a device without room for it stages this member alone
+        std::lock_guard<std::mutex> lock(E->links_mu);
         if (!E->d_links) {
             size_t most = 0;
             for (const EnsMember &m2 : E->members)
                 if (m2.link) most = std::max(most, (size_t)m2.n_vars);
-            e = cudaMalloc((void **)&E->d_links, most);
-            if (e == cudaSuccess) E->allocs.push_back(E->d_links);
+            if (cudaMalloc((void **)&E->d_links, most) != cudaSuccess) {
+                E->d_links = nullptr;
+                (void)cudaGetLastError();
+            }
         }
-        if (e == cudaSuccess) e = launch_planes_to_links(mem.a.state, E->d_links, mem.a.g.n_sites, mem.a.g.d, E->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(out, E->d_links, (size_t)mem.n_vars, cudaMemcpyDeviceToHost, E->stream);
+        uint8_t *own = nullptr;
+        if (!E->d_links) e = cudaMalloc((void **)&own, (size_t)mem.n_vars);
+        uint8_t *links = own ? own : E->d_links;
+        if (e == cudaSuccess) e = launch_planes_to_links(mem.a.state, links, mem.a.g.n_sites, mem.a.g.d, E->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(out, links, (size_t)mem.n_vars, cudaMemcpyDeviceToHost, E->stream);
+        const cudaError_t done = cudaStreamSynchronize(E->stream);  // (before the next call writes the buffer)
+        if (e == cudaSuccess) e = done;
+        if (own) cudaFree(own);
     } else {
         e = cudaMemcpyAsync(out, mem.a.state, (size_t)mem.n_vars, cudaMemcpyDeviceToHost, E->stream);
     }
@@ -1856,6 +1867,7 @@ extern "C" void plq_ensemble_destroy(plq_ensemble *E) {
     if (E->stream) cudaStreamSynchronize(E->stream);
     drop_graph(E);
     for (void *p : E->allocs) cudaFree(p);
+    if (E->d_links) cudaFree(E->d_links);
     if (E->stream) cudaStreamDestroy(E->stream);
     delete E;
 }
