@@ -1899,6 +1899,7 @@ struct ServerJob {
     std::string message;
     double t_submit = 0, t_admit = 0, t_finish = 0;
     uint64_t footprint = 0;
+    uint64_t rows = 0;  // device bytes of its packed rows, beside the footprint
     // device state while active
     EnsMember mem;
     TableSet ts;
@@ -1912,7 +1913,8 @@ struct ServerJob {
 struct plq_server {
     plq_ctx ctx_copy;        // the context's record, copied at creation (outlives the caller's)
     plq_ctx *ctx = nullptr;  // = &ctx_copy
-    uint64_t budget = 0, used = 0;
+    uint64_t budget = 0, used = 0;  // used: the footprints of the admitted jobs, which alone decide admission
+    uint64_t rows = 0;              // what their packed rows take of the rest; given up to jobs that need it
     int max_slots = 0;
     double tick_ms = 10.0;
     std::mutex mu;
@@ -1980,7 +1982,7 @@ cudaError_t job_repack(const ServerJob *j, bool unpack, cudaStream_t stream) {
 }
 
 // Allocate and upload a job's resident state (worker thread, device current).
-int job_admit(ServerJob *j, bool room_for_rows, cudaStream_t stream) {
+int job_admit(ServerJob *j, cudaStream_t stream) {
     const plq_chain_desc &d = j->desc;
     EnsMember &mem = j->mem;
     std::memset(&mem, 0, sizeof mem);
@@ -2016,14 +2018,7 @@ int job_admit(ServerJob *j, bool room_for_rows, cudaStream_t stream) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
         if (e == cudaSuccess) j->allocs.push_back(*p);
     };
-    // q = 2 and gauge jobs stay packed from admission to retirement, where the server's budget
-    // has room for the rows beside the bytes (a job is admitted on its bytes alone)
-    const bool packed = room_for_rows && packed_eligible(d);
-    mem.wpt = tuned_wpt(d, packed);
-    if (packed) {
-        alloc(&mem.pk, packed_bytes(d, mem.n_vars));
-        mem.pk_wide = d.model != PLQ_GAUGE && d.shape[0] > 32 ? 1 : 0;
-    }
+    mem.wpt = tuned_wpt(d, false);
     uint8_t *st = nullptr;
     alloc((void **)&st, (size_t)mem.n_vars);
     a.state = st;
@@ -2044,7 +2039,6 @@ int job_admit(ServerJob *j, bool room_for_rows, cudaStream_t stream) {
             e = cudaMemsetAsync(st, 0, (size_t)mem.n_vars, stream);
         }
     }
-    if (e == cudaSuccess && mem.pk) e = job_repack(j, false, stream);
     if (e == cudaSuccess && d.rng == PLQ_RNG_STREAM) {
         uint64_t slo, shi, ilo, ihi;
         pcg_seed_from_u64(d.seed, slo, shi, ilo, ihi);
@@ -2097,6 +2091,42 @@ int job_admit(ServerJob *j, bool room_for_rows, cudaStream_t stream) {
         return plq_fail(e == cudaErrorMemoryAllocation ? PLQ_ENOMEM : PLQ_ECUDA, cudaGetErrorString(e));
     }
     return PLQ_OK;
+}
+
+// q = 2 and gauge jobs run packed while their rows find a place beside the bytes on which a job
+// is admitted: in what the budget leaves, and on the device.  False: the job runs on its bytes.
+bool job_pack(ServerJob *j, cudaStream_t stream) {
+    EnsMember &mem = j->mem;
+    const uint64_t bytes = packed_bytes(j->desc, mem.n_vars);
+    void *rows = nullptr;
+    cudaError_t e = cudaMalloc(&rows, bytes);
+    if (e == cudaSuccess) {
+        mem.pk = rows;
+        mem.pk_wide = j->desc.model != PLQ_GAUGE && j->desc.shape[0] > 32 ? 1 : 0;
+        e = job_repack(j, false, stream);
+    }
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        if (rows) cudaFree(rows);
+        mem.pk = nullptr;
+        return false;
+    }
+    mem.wpt = tuned_wpt(j->desc, true);
+    j->allocs.push_back(rows);
+    j->rows = bytes;
+    return true;
+}
+
+// An active job goes on on its bytes (between ticks); false: its rows stay.
+bool job_unpack(ServerJob *j, cudaStream_t stream) {
+    EnsMember &mem = j->mem;
+    if (job_repack(j, true, stream) != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess) return false;
+    j->allocs.erase(std::find(j->allocs.begin(), j->allocs.end(), mem.pk));
+    cudaFree(mem.pk);
+    mem.pk = nullptr;
+    mem.wpt = tuned_wpt(j->desc, false);
+    j->rows = 0;
+    return true;
 }
 
 // Device buffers of one tick's launch; grown, never shrunk.
@@ -2262,6 +2292,7 @@ void retire(plq_server *S, ServerJob *j, cudaStream_t stream) {
     job_release(j);
     std::lock_guard<std::mutex> lock(S->mu);
     S->used -= j->footprint;
+    S->rows -= j->rows;
     j->t_finish = now_s();
     if (e != cudaSuccess) {
         j->state = PLQ_JOB_FAILED;
@@ -2298,18 +2329,33 @@ void worker_loop(plq_server *S) {
                 }
             }
         }
-        for (ServerJob *j : admit) {
-            bool rows = false;
-            if (packed_eligible(j->desc)) {  // the packed rows, where the budget has room for them
-                const uint64_t bytes = packed_bytes(j->desc, desc_vars(j->desc));
+        // packed rows make room for the jobs just admitted
+        for (ServerJob *j : S->active) {
+            if (!j->rows) continue;
+            const uint64_t rows = j->rows;
+            {
                 std::lock_guard<std::mutex> lock(S->mu);
-                rows = S->used + bytes <= S->budget;
-                if (rows) {
-                    S->used += bytes;
-                    j->footprint += bytes;
+                if (S->used + S->rows <= S->budget) break;
+            }
+            if (!job_unpack(j, stream)) continue;
+            std::lock_guard<std::mutex> lock(S->mu);
+            S->rows -= rows;
+        }
+        for (ServerJob *j : admit) {
+            int rc = job_admit(j, stream);
+            if (rc == PLQ_OK && packed_eligible(j->desc)) {
+                const uint64_t rows = packed_bytes(j->desc, j->mem.n_vars);
+                bool room;
+                {
+                    std::lock_guard<std::mutex> lock(S->mu);
+                    room = S->used + S->rows + rows <= S->budget;
+                    if (room) S->rows += rows;
+                }
+                if (room && !job_pack(j, stream)) {
+                    std::lock_guard<std::mutex> lock(S->mu);
+                    S->rows -= rows;
                 }
             }
-            int rc = job_admit(j, rows, stream);
             std::lock_guard<std::mutex> lock(S->mu);
             if (rc != PLQ_OK) {
                 S->used -= j->footprint;
@@ -2358,6 +2404,7 @@ void worker_loop(plq_server *S) {
                     j->error = rc;
                     j->message = S->device_message;
                     S->used -= j->footprint;
+                    S->rows -= j->rows;
                 }
             } else if (remaining) {
                 for (ServerJob *j : S->active) {
@@ -2540,7 +2587,7 @@ extern "C" int plq_server_stats(plq_server *S, double *out) {
     out[4] = (double)S->ticks;
     out[5] = (double)S->queue.size();
     out[6] = (double)S->active.size();
-    out[7] = (double)S->used;
+    out[7] = (double)(S->used + S->rows);
     return S->device_error;
 }
 
