@@ -25,9 +25,9 @@
 //               PCG stream: clusters in root order draw next_below(q) (or the
 //               forced-change proposal) at consecutive positions, inside the
 //               rank scan; rand's range sampler occasionally takes a second
-//               draw, which shifts every later cluster -- those rare events
-//               are reported by the scan and fixed up by drawing the labels
-//               again with the events known (settle_labels_kernel).
+//               draw, which shifts every later cluster -- the scan lists the
+//               outputs that do, and the pass that hands the labels to the sites
+//               draws the shifted ones again (SecondDraws).
 //
 // Wolff on the keyed stream: the reference relabels the cluster of a keyed
 // seed site in the full decomposition (cluster_relabel.wgsl:55-66).  Here one
@@ -50,6 +50,7 @@
 #include "plq_geom.cuh"
 #include "plq_local.h"
 #include "plq_readback.h"
+#include "plq_second_draws.h"
 #include "plq_tables.h"
 #include "plq_wolff_sync.h"
 
@@ -62,7 +63,6 @@ constexpr int kSitesPerThread = 8;
 constexpr int kChunk = kThreads * kSitesPerThread;
 constexpr int kSpinLimit = 1 << 22;
 constexpr int kMaxEvents = 64;
-constexpr int kNoEvent = 0x7FFFFFFF;
 constexpr unsigned long long kDescAgg = 1ull, kDescPrefix = 2ull;
 
 struct ClusterArgs {
@@ -91,8 +91,8 @@ struct ClusterArgs {
     uint64_t ticket_base;
     uint32_t epoch;
     int cap;          // iteration cap of finds and unions
-    int32_t *events;  // device: sorted ranks of clusters that take two draws
-    int *first_new;   // device: smallest rank with an unknown second draw; [1]: the number of events
+    int32_t *events;   // stream relabel: label outputs that ask for a second draw (places from the first label)
+    int *event_count;  // ... their number; the list holds the first kMaxEvents
     uint64_t updates; // Wolff: updates in this launch
 };
 
@@ -272,10 +272,7 @@ __global__ void __launch_bounds__(kThreads) bonds_kernel(ClusterArgs a) {
         __shared__ unsigned long long s_base, s_excl0;
         __shared__ u128 s_state;
         if (threadIdx.x == 0) {
-            if (chunk == 0) {  // this sweep's second draws: none known
-                a.first_new[0] = kNoEvent;
-                a.first_new[1] = 0;
-            }
+            if (chunk == 0) *a.event_count = 0;
             s_base = a.ctrl->pos[0];
             if (chunk == a.n_chunks - 1) a.ctrl->pos[1] = s_base + excl + (unsigned long long)total;
             s_excl0 = excl;
@@ -809,7 +806,7 @@ __device__ __forceinline__ int32_t find_root_ro(const int32_t *parent, int32_t x
 
 // A relabel pass over one tile.  The tile's local roots are gathered into a list
 // in shared memory; each walks to its cluster's root once (and stores it, so
-// walks through it end there), and of_root(root) gives the value of its sites;
+// walks through it end there), and of_root(root, the local root) gives the value of its sites;
 // then out takes the sites of each row four at a time.  Bound by the latency of the
 // walks, hence the list: full warps of walks instead of one lane in eight.
 template <class T>
@@ -869,7 +866,7 @@ __device__ __forceinline__ void tile_relabel(const ClusterArgs &a, uint32_t tile
                 root = find_root_ro(a.parent, up[k], a.cap, a.ctrl);
                 if (root != up[k]) a.parent[s[k]] = root;
             }
-            s_value[li[k]] = of_root(root);
+            s_value[li[k]] = of_root(root, s[k]);
         }
     }
     __syncthreads();
@@ -901,7 +898,7 @@ __global__ void __launch_bounds__(kThreads) flatten_kernel(ClusterArgs a) {
     using T = Tile<D, SMALL>;
     __shared__ RelabelShared<T> sm;
     tile_relabel<T>(
-        a, blockIdx.x, sm, [](int32_t) { return (uint8_t)0; },
+        a, blockIdx.x, sm, [](int32_t, int32_t) { return (uint8_t)0; },
         [&](uint32_t s, int count, const uint32_t (&r)[4], const uint8_t *, const T &t, uint32_t s_tile) {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
@@ -918,7 +915,7 @@ __global__ void __launch_bounds__(kThreads) relabel_keyed_kernel(ClusterArgs a) 
     __shared__ RelabelShared<T> sm;
     tile_relabel<T>(
         a, blockIdx.x, sm,
-        [&](int32_t root) {
+        [&](int32_t root, int32_t) {
             // the forced change's step, or the label itself
             const float u = __fmul_rn((float)keyed24(a.seed32 ^ kRootSalt, (uint32_t)root, a.sweep32),
                                       5.9604644775390625e-8f);
@@ -953,17 +950,19 @@ __device__ __forceinline__ uint32_t next_below_from(const ClusterArgs &a, u128 s
 // The fresh label of a cluster (ClusterUpdate::fresh_label, updater.rs:507-521)
 // whose first draw is the output of st: next_below(q), or with forced change the
 // proposal of updater.rs:659-668 (q >= 3 there).
+__device__ __forceinline__ uint32_t label_range(const ClusterArgs &a) {
+    return (uint32_t)(a.relabel == PLQ_RELABEL_REDRAW ? a.q : a.q - 1);
+}
 __device__ __forceinline__ uint32_t fresh_label(const ClusterArgs &a, u128 st, uint32_t cur, bool &second) {
-    if (a.relabel == PLQ_RELABEL_REDRAW) return next_below_from(a, st, (uint32_t)a.q, second);
-    const uint32_t d = next_below_from(a, st, (uint32_t)(a.q - 1), second);
-    return d + (d >= cur ? 1u : 0u);
+    const uint32_t d = next_below_from(a, st, label_range(a), second);
+    return a.relabel == PLQ_RELABEL_REDRAW ? d : d + (d >= cur ? 1u : 0u);
 }
 
 // stream: rank of each root among roots (first-encounter order), and each
-// root's fresh label drawn with no second draws known: rank r draws at
-// bond_end + r, so a thread steps the stream from one root to the next.  A root
-// whose label takes a second draw reports its rank in first_new; settle_labels_kernel
-// then draws the labels again with that event known.
+// root's fresh label as if no label before it took a second draw: rank r draws at
+// bond_end + r, so a thread steps the stream from one root to the next.  Whether an
+// output asks for a second draw is a property of the output alone, so this pass
+// also lists every such place of the stream (SecondDraws resolves them).
 template <int D>
 __global__ void __launch_bounds__(kThreads) root_rank_kernel(ClusterArgs a) {
     const int64_t n = a.g.n_sites;
@@ -996,7 +995,10 @@ __global__ void __launch_bounds__(kThreads) root_rank_kernel(ClusterArgs a) {
     __shared__ u128 s_state;
     __shared__ unsigned long long s_excl0;
     if (threadIdx.x == 0) {
-        if (chunk == a.n_chunks - 1) a.ctrl->scratch[0] = excl + (unsigned long long)total;
+        if (chunk == a.n_chunks - 1) {  // (apply_fresh_kernel adds the second draws)
+            a.ctrl->scratch[0] = excl + (unsigned long long)total;
+            a.ctrl->pos[0] = a.ctrl->pos[1] + excl + (unsigned long long)total;
+        }
         // labels are drawn from the end of the bond draws, in root rank order
         const u128 st0 = jump(a.jump, a.at[1], excl);
         a.chunk_base[chunk].st = st0;
@@ -1005,7 +1007,7 @@ __global__ void __launch_bounds__(kThreads) root_rank_kernel(ClusterArgs a) {
         s_excl0 = excl;
     }
     __syncthreads();
-    // the state after the labels (settle_labels_kernel adds second draws), beside the draws
+    // the state after the labels, beside the draws
     if (chunk == a.n_chunks - 1 && threadIdx.x == kThreads - 1) a.at[0] = jump(a.jump, s_state, (uint64_t)total);
     if (!count) return;
     u128 st = jump(a.jump, s_state, excl - s_excl0);
@@ -1017,83 +1019,73 @@ __global__ void __launch_bounds__(kThreads) root_rank_kernel(ClusterArgs a) {
         a.rank[s] = r;
         bool second;
         a.fresh[s] = (uint8_t)fresh_label(a, st, a.state[s], second);
-        if (second) atomicMin(a.first_new, r);
+        if (second) {
+            const int k = atomicAdd(a.event_count, 1);
+            if (k < kMaxEvents) a.events[k] = r;
+        }
         st = pcg_step(st, a.inc);
         ++r;
     }
 }
 
-// stream, after the rank pass: where a label took a second draw, every label again
-// -- each root draws its cluster's fresh label (ClusterUpdate::fresh_label,
-// updater.rs:507-521) at bond_end + rank + (known second draws before it), jumping
-// from its root_rank chunk's first label draw -- until no unknown second draw
-// turns up; then the stream position after the sweep.  One CTA: such a draw comes
-// once in 2^32 / (q - 1) labels, and a launch that finds none costs less than
-// asking the host (3D Potts q = 3 96^3: 91 us a sweep with the host's answer,
-// 72 so).
-constexpr int kSettleThreads = 256;
-template <int D, bool SMALL>
-__global__ void __launch_bounds__(kSettleThreads) settle_labels_kernel(ClusterArgs a, uint32_t n_tiles) {
-    using T = Tile<D, SMALL>;
-    __shared__ int s_n;
-    volatile int *first_new = a.first_new;
-    for (int n = 0;; ++n) {
-        __syncthreads();
-        const int first = first_new[0];
-        __syncthreads();  // (all have read it)
-        if (first == kNoEvent) {
-            if (threadIdx.x == 0) {
-                a.ctrl->pos[0] = a.ctrl->pos[1] + a.ctrl->scratch[0] + (unsigned long long)n;
-                for (int k = 0; k < n; ++k) a.at[0] = pcg_step(a.at[0], a.inc);
-            }
-            return;
-        }
-        if (n == kMaxEvents) {
-            if (threadIdx.x == 0) atomicOr(&a.ctrl->status, kStatusQueueOverflow);
-            return;
-        }
-        if (threadIdx.x == 0) {  // into the sorted list
-            int k = n;
-            for (; k > 0 && a.events[k - 1] > first; --k) a.events[k] = a.events[k - 1];
-            a.events[k] = first;
-            s_n = n + 1;
-            first_new[0] = kNoEvent;
-            __threadfence();
-        }
-        __syncthreads();
-        const int known_n = s_n;
-        const T t(a.g);
-        for (uint32_t tile = 0; tile < n_tiles; ++tile) {
-            int xt[3];
-            const uint32_t s_tile = t.origin(tile, xt);
-            for (uint32_t li = threadIdx.x; li < T::kSites; li += kSettleThreads) {
-                if (!t.inside(xt, li) || a.local_root[(size_t)tile * T::kSites + li] != li) continue;
-                const int64_t s = t.site(s_tile, li);
-                if (a.parent[s] != (int32_t)s) continue;
-                const int32_t r = a.rank[s];
-                int before = 0;
-                bool known = false;
-                for (int e = 0; e < known_n; ++e) {
-                    before += a.events[e] < r;
-                    known |= a.events[e] == r;
-                }
-                const ClusterArgs::ChunkBase &cb = a.chunk_base[s / kChunk];
-                const u128 st = jump(a.jump, cb.st, (uint64_t)((int64_t)r - cb.rank0) + (uint64_t)before);
-                bool second;
-                a.fresh[s] = (uint8_t)fresh_label(a, st, a.state[s], second);
-                if (second && !known) atomicMin(a.first_new, r);
-            }
-        }
-        __threadfence();
-    }
+// The labels of a sweep that take a second draw (plq_second_draws.h).
+struct SecondDraws {
+    int n;
+    int32_t place[kMaxEvents], rank[kMaxEvents];
+};
+
+// (one thread)  False: more of them than the list holds.
+__device__ __noinline__ bool second_draws(const ClusterArgs &a, int listed, SecondDraws &sd) {
+    for (int i = 0; i < listed && i < kMaxEvents; ++i) sd.place[i] = a.events[i];
+    const int64_t labels = (int64_t)a.ctrl->scratch[0];
+    u128 st = jump(a.jump, a.at[1], (uint64_t)labels);
+    return resolve_second_draws(sd.place, listed, labels, kMaxEvents, sd.rank, sd.n, [&](int64_t) {
+        bool second;
+        next_below_from(a, st, label_range(a), second);
+        st = pcg_step(st, a.inc);
+        return second;
+    });
 }
 
+// The label of a cluster whose draw `before` second draws have moved, `cur` its present state.
+__device__ __noinline__ uint8_t moved_label(const ClusterArgs &a, int32_t root, int32_t rank, int before, uint32_t cur) {
+    const ClusterArgs::ChunkBase &cb = a.chunk_base[root / kChunk];
+    bool second;
+    return (uint8_t)fresh_label(a, jump(a.jump, cb.st, (uint64_t)((int64_t)rank - cb.rank0) + (uint64_t)before), cur, second);
+}
+
+// stream: the labels to the sites, those behind a second draw drawn again (by every tile that
+// meets the cluster), and the position behind the second draws.  A sweep without one, nearly
+// every sweep, pays a load per CTA for it.
 template <int D, bool SMALL>
-__global__ void __launch_bounds__(kThreads) apply_fresh_kernel(ClusterArgs a) {
+__global__ void __launch_bounds__(kThreads, 8) apply_fresh_kernel(const __grid_constant__ ClusterArgs a) {
     using T = Tile<D, SMALL>;
     __shared__ RelabelShared<T> sm;
+    __shared__ SecondDraws sd;
+    const int listed = *a.event_count;
+    if (listed) {
+        if (threadIdx.x == 0) {
+            if (!second_draws(a, listed, sd)) atomicOr(&a.ctrl->status, kStatusQueueOverflow);
+            if (blockIdx.x == 0) {
+                const unsigned long long draws = a.ctrl->scratch[0] + (unsigned long long)sd.n;
+                a.ctrl->pos[0] = a.ctrl->pos[1] + draws;
+                a.at[0] = jump(a.jump, a.at[1], draws);
+            }
+        }
+        __syncthreads();
+    }
     tile_relabel<T>(
-        a, blockIdx.x, sm, [&](int32_t root) { return a.fresh[root]; },
+        a, blockIdx.x, sm,
+        [&](int32_t root, int32_t s) {
+            if (listed) {
+                const int32_t rank = a.rank[root];
+                int before = 0;
+                for (int k = 0; k < sd.n; ++k) before += sd.rank[k] < rank;
+                // (a cluster's sites agree, and this CTA alone writes its own)
+                if (before) return moved_label(a, root, rank, before, a.state[s]);
+            }
+            return a.fresh[root];
+        },
         [&](uint32_t s, int count, const uint32_t (&r)[4], const uint8_t *value, const T &, uint32_t) {
             const uint8_t v[4] = {value[r[0]], value[r[1]], value[r[2]], value[r[3]]};
             store_row(a.state, s, count, v);
@@ -1350,7 +1342,7 @@ wolff_kernel(ClusterArgs a, WolffSync *w, uint32_t n_tiles, unsigned long long l
         RelabelShared<T> &sm = *reinterpret_cast<RelabelShared<T> *>(s_buf);
         for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
             tile_relabel<T>(
-                a, tile, sm, [&](int32_t r) { return (uint8_t)(r == root ? 1 : 0); },
+                a, tile, sm, [&](int32_t r, int32_t) { return (uint8_t)(r == root ? 1 : 0); },
                 [&](uint32_t s, int count, const uint32_t (&r)[4], const uint8_t *value, const T &, uint32_t) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
@@ -1434,7 +1426,7 @@ struct ClusterDev {
     int64_t n_tiles = 0;  // CTAs of the kernels that take a tile each
     bool small_tiles = false;
     int32_t *events = nullptr;
-    int *first_new = nullptr;
+    int *event_count = nullptr;
     int32_t *sizes = nullptr;
     uint32_t kp24 = 0;
     uint64_t kp53 = 0;
@@ -1477,7 +1469,7 @@ ClusterArgs cluster_args(plq_chain *c) {
     a.n_chunks = cd->n_chunks;
     a.cap = (c->desc.flags & PLQ_FLAG_TINY_PASS_CAP) ? 1 : (int)std::min<int64_t>(c->n_sites + 64, 1 << 30);
     a.events = cd->events;
-    a.first_new = cd->first_new;
+    a.event_count = cd->event_count;
     return a;
 }
 
@@ -1495,9 +1487,6 @@ struct TileKernels {
     }
     static void relabel_keyed(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
         relabel_keyed_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
-    }
-    static void settle(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
-        settle_labels_kernel<D, SMALL><<<1, kSettleThreads, 0, st>>>(a, tiles);
     }
     static void apply_fresh(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
         apply_fresh_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
@@ -1562,11 +1551,10 @@ int sweep_t(plq_chain *c, uint64_t sweeps) {
             c->launches++;
         } else {
             lookback(a);
-            // ranks, and the labels with no second draws known; the second draws; the labels to the sites
+            // ranks, and the labels with no second draws known; the labels to the sites
             root_rank_kernel<D><<<(unsigned)cd->n_chunks, kThreads, 0, c->stream>>>(a);
-            K::settle(a, (unsigned)cd->n_tiles, c->stream);
             K::apply_fresh(a, (unsigned)cd->n_tiles, c->stream);
-            c->launches += 3;
+            c->launches += 2;
         }
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return plq_fail(PLQ_ECUDA, std::string("cluster sweep: ") + cudaGetErrorString(e));
@@ -1669,7 +1657,7 @@ int cluster_create(plq_chain *c) {
             alloc((void **)&cd->rank, sizeof(int32_t) * (size_t)n);
             alloc((void **)&cd->chunk_base, sizeof(ClusterArgs::ChunkBase) * (size_t)cd->n_chunks);
             alloc((void **)&cd->events, sizeof(int32_t) * kMaxEvents);
-            alloc((void **)&cd->first_new, 2 * sizeof(int));
+            alloc((void **)&cd->event_count, sizeof(int));
             alloc((void **)&cd->at, 2 * sizeof(u128));
             if (e == cudaSuccess) e = cudaMemcpyAsync(cd->at, &c->base, sizeof(u128), cudaMemcpyHostToDevice, c->stream);
         }
@@ -1700,7 +1688,7 @@ void cluster_free(plq_chain *c) {
     ClusterDev *cd = static_cast<ClusterDev *>(c->cl);
     if (!cd) return;
     void *ptrs[] = {cd->bonds, cd->parent, cd->local_root, cd->fresh, cd->rank, cd->chunk_base, cd->wolff, cd->at,
-                    cd->desc, cd->events, cd->first_new, cd->sizes};
+                    cd->desc, cd->events, cd->event_count, cd->sizes};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     delete cd;
