@@ -58,8 +58,8 @@ WORKLOADS = {
                               "stream, uniform random start from seed 20260718", "fused3d_kernel<2,false,false>", 1),
     "ising-512-metro-stream": ("ising", 2, "metropolis", "stream", 0.2216544,
                                "3D Ising 512^3 periodic, checkerboard Metropolis, beta=0.2216544, PCG64 reference "
-                               "stream (bit-exact with the reference CPU path; device-wide scan per colour pass), "
-                               "uniform random start from seed 20260718", "scan_metro_kernel<3>", 2),
+                               "stream (bit-exact with the reference CPU path; device-wide count of the draws per "
+                               "colour pass), uniform random start from seed 20260718", "scan_metro_kernel<3>", 2),
 }
 
 
@@ -272,7 +272,7 @@ def measure_local(name, steps, warmup, ctx, e2e=True):
     dev_ms = ev0.elapsed_time(ev1)
     clock_info = clocks.stop(t_wall0, t_wall1)
     chain.sync()
-    path = chain.path
+    path, resident = chain.path, chain.resident
     chain.close()
     dev_ms_max = max_over_ranks(pg, dev_ms, local)
     barrier(pg, local)
@@ -290,8 +290,14 @@ def measure_local(name, steps, warmup, ctx, e2e=True):
         l2_note = ("134 MB byte state read (packed) and written (unpacked) once per advance call; the sweeps run "
                    "on a 16.8 MB bit-packed copy that stays in L2 and stream each site's 4-byte first keyed hash "
                    "(537 MB, larger than L2) from HBM once per sweep")
-    per_launch_ms = dev_ms / max(1, steps * per_sweep)
-    alg_bytes = BYTES_PER_UPDATE * N_SITES // per_sweep  # per launch of the dominant kernel
+    passes = max(1, steps * per_sweep)  # launches of the dominant kernel
+    if resident:
+        # every sweep of the timed call in one launch, on words of one bit a site
+        kernel, passes = "stream_kernel" if w[3] == "stream" else "resident_kernel", launches
+        l2_note = ("134 MB byte state read (packed) and written (unpacked) once per advance call; the sweeps run "
+                   "on a 16.8 MB bit-packed copy that stays in L2")
+    per_launch_ms = dev_ms / passes
+    alg_bytes = BYTES_PER_UPDATE * N_SITES * steps // passes  # per launch of the dominant kernel
     achieved = alg_bytes / (per_launch_ms * 1e-3) / 1e9
     peak, peak_kind = measured_peak_hbm()
     traffic, traffic_src = traffic_record(name, kernel)
@@ -301,7 +307,7 @@ def measure_local(name, steps, warmup, ctx, e2e=True):
         "scaling": "weak", "vs_baseline": None, "dtype": "u8", "data": "synthetic",
         "config": {"workload": w[5], "name": name, "sites_per_gpu": N_SITES, "step": "one sweep",
                    "l2": l2_note,
-                   "parallelism": f"independent lattice per GPU x{world}", "path": path},
+                   "parallelism": f"independent lattice per GPU x{world}", "path": path, "resident": resident},
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "traffic": traffic, "traffic_source": traffic_src,
                      "peak_source": peak_kind, "algorithmic_bytes_per_launch": alg_bytes, "kernel": kernel,
@@ -667,8 +673,7 @@ CLUSTER_WORKLOADS = {
                        "2D Ising 4096^2 periodic Swendsen-Wang, beta=0.4406868, PCG64 reference stream (bit-exact "
                        "with the reference CPU ClusterUpdate), uniform random start"),
     "wolff-128-keyed": ("seeded", "keyed", (128, 128, 128), 0.2216544,
-                        "3D Ising 128^3 periodic Wolff (keyed seed site, frontier BFS), beta=0.2216544, uniform "
-                        "random start"),
+                        "3D Ising 128^3 periodic Wolff (keyed seed site), beta=0.2216544, uniform random start"),
 }
 
 
@@ -746,7 +751,8 @@ def measure_cluster(name, steps, warmup, ctx, e2e=True):
                       "kernel": "bonds + tile union-find + boundary unions + relabel",
                       "note": "10.5 B/site per sweep algorithmic minimum"} if not wolff else
                      {"bound": "latency", "achieved": None, "peak": None, "unit": None, "frac": None,
-                      "traffic": None, "note": "frontier BFS: work proportional to the cluster, not the lattice"}),
+                      "traffic": None, "note": "growth from the seed site for a small cluster, labelling of the lattice's "
+                                              "tiles for a large one; barriers and a row's chain of labels"}),
         "size_histogram_log2": [int(x) for x in hist[:24]],
         "gpu_launches": launches,
         "clocks": clock_info,

@@ -76,7 +76,9 @@ enum plq_rng { PLQ_RNG_STREAM = 0, PLQ_RNG_KEYED = 1 };
 /* Bit-packed chains only: hash both keyed rounds in every pass instead of
  * reading each site's sweep-independent first round from the array filled at
  * creation (identical results; used to test the hashing passes, which also
- * serve lattices of 2^31 sites and more and chains whose array found no room). */
+ * serve lattices of 2^31 sites and more and chains whose array found no room).
+ * This flag and the three that name a pass (NO_FUSED, GENERIC_PASS, NO_PACKED)
+ * also give every pass its own launch, on every chain (plq_chain_resident). */
 #define PLQ_FLAG_NO_FIRST_HASH 32
 
 typedef struct plq_ctx plq_ctx;
@@ -196,10 +198,16 @@ int plq_chain_cluster_labels(plq_chain *chain, int32_t *out);
  * clusters with 2^k <= size < 2^(k+1) (the last bin takes the rest).  Wolff
  * chains: the cluster of the most recent update. */
 int plq_chain_cluster_histogram(plq_chain *chain, int64_t *hist, int32_t nbins);
-/* Which device path the chain's sweeps take: "fused3d" (both colours in one
- * pass), "pass" (one launch per colour), "lookback" (stream Metropolis with
- * the device-wide scan), "cluster". */
+/* Which form the chain's passes take: "fused3d" (both colours in one pass),
+ * "packed" (keyed q = 2 sites whose rows are whole 64-site words, one bit a
+ * site), "words" (four sites at a time), "pass" (one variable at a time),
+ * "lookback" (stream Metropolis, whose draws' places depend on the states),
+ * "cluster". */
 const char *plq_chain_path(plq_chain *chain);
+/* 1 if the sweeps of a call run in one launch with a barrier per pass (q = 2
+ * chains on packed words then, whatever plq_chain_path names), 0 if each pass
+ * is a launch. */
+int plq_chain_resident(plq_chain *chain);
 /* Kernels this chain has launched so far. */
 uint64_t plq_chain_launches(plq_chain *chain);
 void plq_chain_destroy(plq_chain *chain);

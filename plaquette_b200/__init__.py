@@ -111,6 +111,7 @@ _SIGNATURES = {
     "plq_chain_cuda_stream": ([C.c_void_p], C.c_void_p),
     "plq_chain_launches": ([C.c_void_p], C.c_uint64),
     "plq_chain_path": ([C.c_void_p], C.c_char_p),
+    "plq_chain_resident": ([C.c_void_p], C.c_int),
     "plq_chain_axis_pair_sums": ([C.c_void_p, C.c_void_p, C.c_int64], C.c_int),
     "plq_chain_polyakov": ([C.c_void_p, C.c_int32, C.POINTER(C.c_int64), C.POINTER(C.c_int64)], C.c_int),
     "plq_chain_wilson": ([C.c_void_p, C.c_int32, C.c_void_p, C.c_int64, C.POINTER(C.c_int64),
@@ -362,6 +363,10 @@ class GpuChain:
     @property
     def path(self) -> str:
         return lib().plq_chain_path(self._h).decode()
+
+    @property
+    def resident(self) -> bool:
+        return bool(lib().plq_chain_resident(self._h))
 
     @property
     def launches(self) -> int:

@@ -1128,4 +1128,5 @@ extern "C" const char *plq_chain_path(plq_chain *c) {
     if (c->packed) return "packed";
     return c->lookback ? "lookback" : (c->words ? "words" : "pass");
 }
+extern "C" int plq_chain_resident(plq_chain *c) { return c && c->resident.kind != ResidentKind::kNone ? 1 : 0; }
 extern "C" void plq_chain_destroy(plq_chain *c) { chain_free(c); }
