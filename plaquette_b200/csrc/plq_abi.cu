@@ -330,18 +330,63 @@ int32_t first_bad_start(int32_t n, const uint8_t *const *starts, const int64_t *
     return (int32_t)m;
 }
 
+// Whether a q = 2 chain's packed words or rows, sizes at which their passes fill the chip, are
+// faster resident than the per-pass kernels on bytes (below: us a sweep, per-pass / resident).
+// A thread's cost per word hardly depends on how many sites the word holds, so rows that fill
+// little of a word lose, and so do rows of several words whose last one is short (a warp waits
+// for its full ones).  The lines follow from sweeps over extents 0 of 2 .. 1040 and 2^15 .. 2^25
+// variables; where the bytes go four (or, Metropolis on the PCG stream, 16) at a time they
+// are the faster side at smaller sizes than where they go one by one.
+static bool packed_words_pay(const plq_chain_desc &d, int L0, int64_t n_sites, const ResidentPlan &p) {
+    const bool metropolis = d.updater == PLQ_METROPOLIS, stream = d.rng == PLQ_RNG_STREAM;
+    const int64_t units = p.units, word_sites = 64 * (int64_t)p.words_per_row;
+    auto below = [&](int log2) { return units < (int64_t(1) << log2); };
+    if (d.model == PLQ_GAUGE) {
+        // 2D 2 x 2^20 Metropolis 96 / 162, 4 x 2^19 97 / 106; heat bath 4 x 2^18 33 / 37, 2 x 2^19
+        // 45 / 63, 8 x 2^19 66 / 71; 3D 4 x 1024^2 heat bath 120 / 171; keyed 2D 4 x 2^20 41 / 44
+        if (!stream) return L0 != 4 || below(20);
+        if (metropolis) return L0 > 4 || below(L0 == 4 ? 19 : 18);
+        return L0 == 4 ? below(18) : L0 == 2 || (L0 == 8 && d.d == 2) ? below(19) : true;
+    }
+    if (!stream) {
+        // 8 x 2^19 16.4 / 17.7, 8 x 2^21 45 / 56, 4 x 2^19 12.5 / 15.9, 4 x 2^22 49 / 93, 2 x 2^21
+        // 37 / 45; one size below 12.3 / 11.1, 12.3 / 10.1, 23 / 24; 72 x 233016 45 / 52
+        if (L0 == 4 || L0 == 8) return below(19);
+        if (L0 == 2) return below(20);
+        return L0 % 4 != 0 || 4 * word_sites < 7 * L0 || n_sites < (int64_t(1) << 23);
+    }
+    if (!metropolis) {
+        // 4 x 2^17 12.4 / 13.2, 4 x 2^22 90 / 216, 8 x 2^18 20.5 / 21.7, 2 x 2^19 20.6 / 34
+        return L0 == 4 || L0 == 8 ? units < (int64_t)L0 << 15 : L0 != 2 || below(19);
+    }
+    if (L0 % 16 == 0) {
+        // 16 x 2^17 24.6 / 26.8 (2^16: 16.9 / 14.5), 32 x 2^17 28.7 / 31.4, 48 x 174762 49 / 58;
+        // 80 x 104856 49 / 66, 96 x 10922 16.9 / 18.7, 208 x 40328 49 / 66; 112, 176, 240 and more, and
+        // whole words: resident (2^23 sites 49 / 39 .. 43)
+        if (p.words_per_row == 1) return L0 == 64 || n_sites < (int64_t(1) << 20) << (L0 / 16);
+        return 5 * word_sites < 6 * L0 || n_sites < (int64_t(1) << 20);
+    }
+    return L0 >= 8 || units < 5 * 32768;  // 2 x 2^18 30 / 40, 4 x 2^18 37 / 40, 6 x 174762 36.9 / 40.9
+}
+
 // The lattices that run resident: where a barrier is cheaper than a launch and
 // the body at least as fast as the per-pass kernel's.
-//  * packed kinds: always (250^3 Ising, whose rows are no multiple of 64 sites, 124 -> 33 us
-//    a sweep), but for rows of whole 64-site words from 2^23 sites on, where the passes that
-//    stream each site's first hash from memory win (256^3: 25.0 us a sweep against 27.2;
-//    4096 x 2048: 16.7 against 16.1);
+//  * packed kinds: while a launch's threads hold a pass at once, always (64^2 Ising 8.2 -> 1.05 us
+//    a sweep), beyond that but for the rows of packed_words_pay and keyed rows of whole 64-site
+//    words from 2^24 sites on, where the passes that stream each site's first hash from memory win (us a sweep,
+//    passes / resident: 2048^2 12.3 / 8.0, 4096 x 2048 16.3 / 13.0, 256 x 192 x 192 16.4 / 13.8;
+//    256^3 24.6 / 24.3, heat bath 24.0 / 24.7; 320^3 37.9 / 45.8, 8192^2 61 / 77);
 //  * one keyed site per thread: always;
-//  * words and ranks: up to one wave of CTAs (400 x 400 x 100 Potts on the PCG stream, several
-//    waves: 131 us a sweep resident, 111 with a launch per pass).
-static bool resident_wanted(const ResidentPlan &p, int64_t n_sites, bool whole_words) {
+//  * words and the generic body: up to one wave of CTAs (400 x 400 x 100 Potts on the PCG stream,
+//    several waves: 131 us a sweep resident, 111 with a launch per pass).
+static bool resident_wanted(const ResidentPlan &p, const plq_chain_desc &d, const int32_t *L, int64_t n_sites,
+                            bool whole_words) {
     switch (p.kind) {
-        case ResidentKind::kSites: return !(whole_words && n_sites >= (int64_t(1) << 23));
+        case ResidentKind::kSites:
+            if (whole_words) return n_sites < (int64_t(1) << 24);
+            return packed_words_pay(d, L[0], n_sites, p);
+        case ResidentKind::kLinks32:
+        case ResidentKind::kLinks64: return packed_words_pay(d, L[0], n_sites, p);
         case ResidentKind::kWords:
         case ResidentKind::kGeneric: return p.chunks <= p.grid;
         default: return p.kind != ResidentKind::kNone;
@@ -500,7 +545,7 @@ extern "C" int plq_chain_create(plq_ctx *ctx, const plq_chain_desc *desc, const 
                                   plan);
                 if (e != cudaSuccess) return fail(cuda_fail(e, "resident launch plan"));
             }
-            if (resident_wanted(plan, c->n_sites, c->packed)) {
+            if (resident_wanted(plan, *desc, c->g.L, c->n_sites, c->packed)) {
                 c->resident = plan;
                 c->resident_totals = (plan.packed_bytes + 15) & ~(size_t)15;
                 if (plan.packed_bytes)
