@@ -93,7 +93,7 @@ pair_differ_kernel(const uint8_t *cfg, Geom g, const int32_t *pair_mu, const int
 // every displacement of them: one xor and population count per 64 pairs, which
 // is what bounds it.  us per call (about 40 of them
 // the call's copies and synchronisation): 256^3 Ising 3683 -> 155, 1024^2 605 -> 100,
-// 100^3 130 -> 62, 64^3 60 -> 53.
+// 100^3 130 -> 62.  Smaller lattices, and long thin ones, stay with the scan (pair_planes_pay).
 
 // Word w of row r, plane p at words[p * rows * wpr + r * wpr + w]; bits past the row are 0.
 template <int P>
@@ -367,8 +367,25 @@ static size_t pair_shared(const Geom &g, int mu, int planes, uint32_t inner, uin
     return bytes();
 }
 
+// Whether the planes are the faster count.  Both sides from 57 shapes at q = 2, 3, 5 (us a call
+// beyond the 40 of either): the scan makes 1.5 M pairs a us; the planes take 15 for their
+// launches, a chain of steps along each axis past the first (0.014 + 0.0165 a plane a step: a
+// thread walks a line) and 1 M words a us with one plane, 0.5 M with three.  Scan / planes:
+// 8^4 39 / 52, 64^2 40 / 47, 128^2 44 / 48, 300 x 200 49 / 54, 4 x 4096 86 / 169, 2 x 2048 64 / 115
+// (q = 5: 185), 64 x 2048 128 / 123 (184); 80^3 77 / 59, 384^2 76 / 61 (q = 5: 80).
+static bool pair_planes_pay(const Geom &g, int planes) {
+    const double n = (double)g.n_sites, words = n / g.L[0] * ((g.L[0] + 63) / 64);
+    double displacements = 0, steps = 0;
+    for (int mu = 0; mu < g.d; ++mu) {
+        displacements += g.L[mu] / 2;
+        if (mu) steps += g.L[mu];
+    }
+    return n * displacements / 1.5e6 >
+           15 + steps * (0.014 + 0.0165 * planes) + words * displacements * (planes + 1) / 2 / 1e6;
+}
+
 size_t pair_words_bytes(const Geom &g, int q) {
-    if (q > 8 || g.d < 1) return 0;
+    if (q > 8 || g.d < 1 || !pair_planes_pay(g, pair_planes(q))) return 0;
     const int planes = pair_planes(q);
     uint32_t inner = (uint32_t)(g.L[0] + 63) / 64;
     const size_t words = (size_t)(g.n_sites / g.L[0]) * inner;

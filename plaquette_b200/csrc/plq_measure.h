@@ -13,8 +13,8 @@ int64_t pair_sum_entries(const Geom &g);
 cudaError_t launch_pair_differ(const uint8_t *cfg, const Geom &g, const int32_t *pair_mu, const int32_t *pair_r,
                                int n_pairs, long long *out, cudaStream_t stream);
 // The same counts (every axis's displacements 1 .. L/2 in order) from bit planes
-// packed into `words`; pair_words_bytes of scratch, 0 where they do not take the
-// lattice (more than 8 states, an axis too long).
+// packed into `words`; pair_words_bytes of scratch, 0 where the planes do not take the
+// lattice (more than 8 states, an axis too long) or are not the faster count.
 size_t pair_words_bytes(const Geom &g, int q);
 cudaError_t launch_pair_bits(const uint8_t *cfg, const Geom &g, int q, uint64_t *words, int n_pairs, long long *out,
                              int sm_count, cudaStream_t stream);
