@@ -957,21 +957,17 @@ void resident_config(const ResidentPlan &p, cudaLaunchConfig_t &cfg, cudaLaunchA
 constexpr bool packed_kind(ResidentKind k) {
     return k == ResidentKind::kSites || k == ResidentKind::kLinks32 || k == ResidentKind::kLinks64;
 }
-// Attributes of the kernel a plan names, and whether the device takes its cluster.
-template <ResidentKind K, Share S>
+// Whether the device takes the plan's cluster of kGroups CTAs.
+template <ResidentKind K>
 bool cluster_fits(const ResidentPlan &p) {
-    auto kern = resident_kernel<K, S>;
-    cudaError_t e = cudaSuccess;
-    if (p.shared_bytes > 40 * 1024)
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.shared_bytes);
-    int clusters = 1;
-    if (e == cudaSuccess && p.grid > 8) {  // beyond the portable size
-        cudaLaunchConfig_t cfg{};
-        cudaLaunchAttribute attr{};
-        resident_config(p, cfg, attr, nullptr);
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
-    }
+    if (p.grid <= 8) return true;  // the portable size
+    auto kern = resident_kernel<K, kGroups>;
+    int clusters = 0;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    resident_config(p, cfg, attr, nullptr);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
     if (e != cudaSuccess) (void)cudaGetLastError();
     return e == cudaSuccess && clusters > 0;
 }
@@ -997,16 +993,15 @@ cudaError_t plan_kind(ResidentPlan &p, int sm_count) {
                 p.share = kLocal;
                 p.grid = 1;
                 p.block = (int)warps * 32;
-                p.shared_bytes = p.packed_bytes;
-                if (cluster_fits<K, kLocal>(p)) return cudaSuccess;
-                p.shared_bytes = 0;
+                p.shared_bytes = p.packed_bytes;  // (at most 8 KB: 512 rows of four directions)
+                return cudaSuccess;
             }
             p.share = kGroups;
             if (items <= kClusterCtas * kResidentThreads) {
                 p.grid = power_of_two_at_least((warps + 3) / 4);  // at least four warps a CTA
                 if (p.grid > kClusterCtas) p.grid = kClusterCtas;
                 p.block = (int)((warps + p.grid - 1) / p.grid) * 32;
-                if (cluster_fits<K, kGroups>(p)) return cudaSuccess;
+                if (cluster_fits<K>(p)) return cudaSuccess;
             }
             p.cluster = false;
             p.block = kGridThreads;
@@ -1057,9 +1052,8 @@ cudaError_t plan_stream(ResidentPlan &p, int sm_count) {
         p.groups = p.most_groups;
         p.grid = 1;
         p.block = (int)((items + 31) / 32 * 32);
-        p.shared_bytes = p.packed_bytes;
-        if (p.shared_bytes <= 40 * 1024) return cudaSuccess;
-        p.shared_bytes = 0;
+        p.shared_bytes = p.packed_bytes;  // (at most 8 KB, as above)
+        return cudaSuccess;
     }
     p.block = kGridThreads;
     if (items <= (uint32_t)sm_count * 2 * kGridThreads) {
