@@ -42,6 +42,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/plaquette.h"
@@ -95,6 +96,27 @@ struct ClusterArgs {
     int *event_count;  // ... their number; the list holds the first kMaxEvents
     uint64_t updates; // Wolff: updates in this launch
 };
+
+// The launches of a Swendsen-Wang sweep follow each other without a gap: each may take its
+// place on the SMs once the one before has started everywhere (programmatic dependent
+// launch), and waits here for its end.
+__device__ __forceinline__ void after_previous() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+template <class... P, class... A>
+void launch_next(void (*kernel)(P...), unsigned grid, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = stream;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kernel, args...);  // (the sweep asks for the last error)
+}
 
 __device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long *p) {
     unsigned long long v;
@@ -205,6 +227,7 @@ __device__ __forceinline__ uint64_t bytes_equal(uint64_t a, uint64_t b) {
 
 template <int D, bool STREAM>
 __global__ void __launch_bounds__(kThreads) bonds_kernel(ClusterArgs a) {
+    after_previous();
     const int64_t n = a.g.n_sites;
     const int64_t chunk = take_chunk(a, STREAM);
     if (chunk >= a.n_chunks) {
@@ -377,13 +400,18 @@ __device__ __forceinline__ void unite(int32_t *parent, int32_t a, int32_t b, int
 // 0.41 -> 0.196 ms).  The block's 16 rows: 32 had fewer edges but its lists and
 // parents left 4 CTAs per SM (0.215 ms), 8 more boundary unions (0.217 ms).
 //
-// SMALL: fewer rows per block, for lattices that give the large tiles' CTAs to
-// less than two per SM (large_tiles): a block's rows are a serial chain.
-template <int D, bool SMALL>
+// kSmall: fewer rows per block, for lattices that give the large tiles' CTAs to
+// less than two per SM (large_tiles): a block's rows are a serial chain.  kNarrow
+// and kWide stack the blocks along y or x, for lattices short along the other one.
+// kFlat: a run of consecutive sites, for lattices that fill no block (tile_shape).
+enum TileShape { kLarge, kSmall, kNarrow, kWide, kFlat };
+
+template <int D, int SHAPE>
 struct Tile {  // block (per warp): 32 x BY x BZ; tile: WX x WY x WZ blocks
-    static constexpr int BY = D == 1 ? 1 : D == 2 ? (SMALL ? 8 : 16) : (SMALL ? 2 : 4), BZ = D >= 3 ? (SMALL ? 2 : 4) : 1;
-    static constexpr int WX = D == 1 ? 8 : D == 2 ? 4 : (SMALL ? 1 : 2), WY = D == 1 ? 1 : D == 2 || !SMALL ? 2 : 4,
-                         WZ = D >= 3 ? 2 : 1;
+    static constexpr bool kTall = SHAPE == kLarge || SHAPE == kNarrow;
+    static constexpr int BY = D == 1 ? 1 : D == 2 ? (kTall ? 16 : 8) : (kTall ? 4 : 2), BZ = D >= 3 ? BY : 1;
+    static constexpr int WX = D == 1 || SHAPE == kWide ? 8 : D == 2 ? (SHAPE == kNarrow ? 1 : 4) : (SHAPE == kLarge ? 2 : 1),
+                         WZ = D >= 3 && SHAPE != kWide ? 2 : 1, WY = 8 / (WX * WZ);
     static constexpr int TX = 32 * WX, TY = BY * WY, TZ = BZ * WZ;
     static constexpr int kSites = TX * TY * TZ;
     static constexpr int kDims = D;
@@ -436,10 +464,76 @@ struct Tile {  // block (per warp): 32 x BY x BZ; tile: WX x WY x WZ blocks
     }
 };
 
+// Consecutive sites, whatever directions they run along: the places are the sites in
+// order, every bond between two of them is a bond of the tile, periodic ones too.
+template <int D>
+struct Tile<D, kFlat> {
+    static constexpr int TX = 2048, kSites = 2048, kDims = D;
+
+    int32_t L[1];
+    uint32_t n;
+    __host__ __device__ explicit Tile(const Geom &g) : n((uint32_t)g.n_sites) { L[0] = (int32_t)n; }
+    __host__ __device__ int64_t tiles(int64_t n_sites) const { return (n_sites + kSites - 1) / kSites; }
+    __device__ uint32_t origin(uint32_t b, int *x) const {
+        x[0] = (int)(b * kSites);
+        return b * kSites;
+    }
+    __device__ uint32_t site(uint32_t s0, uint32_t li) const { return s0 + li; }
+    __device__ bool inside(const int *x, uint32_t li) const { return (uint32_t)x[0] + li < n; }
+    __device__ uint32_t local_root(const uint16_t *roots, uint32_t s, const int32_t *) const {
+        return s / kSites * kSites + roots[s];
+    }
+};
+
 // Whether the large tiles give every SM two CTAs.
 template <int D>
 bool large_tiles(const Geom &g, int sm_count) {
-    return D >= 2 && Tile<D, false>(g).tiles(g.n_sites) >= 2 * (int64_t)sm_count;
+    return D >= 2 && Tile<D, kLarge>(g).tiles(g.n_sites) >= 2 * (int64_t)sm_count;
+}
+
+// The tiles of a lattice (us a keyed sweep on each):
+//  * flat where the lattice is one of them, so that all bonds lie inside and the boundary launch
+//    falls away (8^2 7 against 13 with kSmall, 32^2 13 / 15; 40^2 17 / 16), and where rows of a few
+//    sites would leave most lanes of a block idle (2 x 2^20 61 / 247 kNarrow, 4 x 65536 27 / 37, 8 x
+//    65536 32 / 38, 12 x 65536 39 / 40; 2 x 2 x 65536 30 / 156 kSmall, 4 x 256 x 256 35 / 46; 8 x 256 x 256
+//    46 / 49 keyed, 76 / 72 on the PCG stream);
+//  * kNarrow for rows up to 96, which overhang the other 2D tiles' 128 columns (32 x 2^19 161 against 515
+//    with kLarge, 96 x 65536 73 / 88), from the sizes on that fill the chip (28 x 8192 25 both; 34 x
+//    4096 26 against 23 with kSmall);
+//  * kWide and kSmall for lattices of few rows, which leave a block's other rows idle (2^21 x 8 204 / 290 /
+//    285 with kWide / kSmall / kLarge, 2^20 x 16 212 / 193 / 220; 65536 x 2 x 2 26 / 36 / 35, 512 x 512 x 2
+//    32 / 30 / 36);
+//  * kSmall for 3D rows up to 32, half of kLarge's (30 x 200 x 200 49 / 64).
+template <int D>
+TileShape fastest_tiles(const Geom &g, int sm_count, bool keyed) {
+    const int64_t n = g.n_sites;
+    if (D == 1) return kSmall;
+    if (n <= 1024) return kFlat;
+    if (D == 2) {
+        if (g.L[0] <= 8 && n >= 32768) return kFlat;
+        if (g.L[0] <= 96 && Tile<D, kSmall>(g).tiles(n) >= 4 * (int64_t)sm_count) return kNarrow;
+        if (g.L[1] <= 8 && n >= (int64_t(1) << 20)) return kWide;
+        if (g.L[1] <= 16) return kSmall;
+    } else {
+        if (g.L[0] <= 4 || (g.L[0] <= 8 && keyed && n >= (int64_t(1) << 18))) return kFlat;
+        if (g.L[1] <= 2 && g.L[2] <= 4) return kWide;
+        if (g.L[0] <= 32 || g.L[2] <= 4) return kSmall;
+    }
+    return large_tiles<D>(g, sm_count) ? kLarge : kSmall;
+}
+
+// ... but flat ones for a lattice of 2^20 sites and more that would have over eight places (2 B each)
+// a site: tubes such as 5 x 1 x 1 x N.
+template <int D>
+TileShape tile_shape(const Geom &g, int sm_count, bool keyed) {
+    const TileShape shape = fastest_tiles<D>(g, sm_count, keyed);
+    const int64_t n = g.n_sites;
+    auto overhangs = [&](auto t) { return t.tiles(n) * t.kSites > 8 * n; };
+    const bool far = shape == kLarge    ? overhangs(Tile<D, kLarge>(g))
+                     : shape == kNarrow ? overhangs(Tile<D, kNarrow>(g))
+                     : shape == kWide   ? overhangs(Tile<D, kWide>(g))
+                                        : overhangs(Tile<D, kSmall>(g));
+    return D >= 2 && n >= (int64_t(1) << 20) && shape != kFlat && far ? kFlat : shape;
 }
 
 // The keyed bond draw of one sweep as an open-draw comparison (plq_packed.cuh):
@@ -510,12 +604,101 @@ struct LabelShared {
     int32_t p[T::kSites];
     uint16_t further[kThreads / 32][kFurther];
 };
+template <int D>
+struct LabelShared<Tile<D, kFlat>> {
+    int32_t p[Tile<D, kFlat>::kSites];
+};
+
+// label_tile for consecutive sites, a thread's a CTA's width apart.  A site first takes as its
+// parent the lowest site of the tile that an open bond leads to it from (an atomic
+// minimum, no find), which makes a forest of long chains along the lattice's long
+// direction; pointer jumping flattens it (united bond by bond instead, every find
+// would walk those chains); the bonds that made no parent are then united.
+template <int D, bool KEYED>
+__device__ __forceinline__ void label_flat(const ClusterArgs &a, uint32_t sweep, uint32_t tile, int32_t *p) {
+    using T = Tile<D, kFlat>;
+    constexpr int S = T::kSites / kThreads;
+    static_assert(S * D <= 64, "a bit per bond of a thread's sites");
+    const uint32_t s0 = tile * T::kSites, here = min((uint32_t)T::kSites, (uint32_t)a.g.n_sites - s0);
+    const int cap = a.cap < T::kSites + 64 ? a.cap : T::kSites + 64;
+    const BondCut cut(a, sweep);
+    const bool bonds = !KEYED || BondCut::some(a);
+    for (uint32_t li = threadIdx.x; li < here; li += kThreads) p[li] = (int32_t)li;
+    __syncthreads();
+    auto neighbours = [&](uint32_t li, uint32_t (&lb)[D]) {
+        int32_t x[D];
+        site_coords<D>(a.g, s0 + li, x);
+#pragma unroll
+        for (int mu = 0; mu < D; ++mu) lb[mu] = (uint32_t)nbr_plus(a.g, s0 + li, x, mu) - s0;
+    };
+    uint64_t open = 0;  // bit i * D + mu: the +mu bond of site i, within the tile
+#pragma unroll 2
+    for (int i = 0; i < S; ++i) {
+        const uint32_t li = threadIdx.x + (uint32_t)(i * kThreads);
+        if (li >= here || !bonds) break;
+        uint32_t lb[D];
+        neighbours(li, lb);
+        const uint32_t own = KEYED ? a.state[s0 + li] : a.bonds[s0 + li];
+#pragma unroll
+        for (int mu = 0; mu < D; ++mu) {
+            if (lb[mu] >= here) continue;
+            const bool o = KEYED ? (a.state[s0 + lb[mu]] == own) & cut.open((s0 + li) * (uint32_t)D + (uint32_t)mu)
+                                 : (own >> mu) & 1u;
+            if (!o) continue;
+            open |= 1ull << (i * D + mu);
+            if (lb[mu] > li) atomicMin(&p[lb[mu]], (int32_t)li);
+        }
+    }
+    __syncthreads();
+    // the bonds that made no parent
+#pragma unroll 1
+    for (int i = 0; i < S; ++i) {
+        const uint32_t li = threadIdx.x + (uint32_t)(i * kThreads), mine = (uint32_t)(open >> (i * D)) & ((1u << D) - 1u);
+        if (!mine) continue;
+        uint32_t lb[D];
+        neighbours(li, lb);
+#pragma unroll
+        for (int mu = 0; mu < D; ++mu)
+            if (((mine >> mu) & 1u) && lb[mu] > li && p[lb[mu]] == (int32_t)li) open &= ~(1ull << (i * D + mu));
+    }
+    __syncthreads();
+    for (bool moved = true; moved;) {  // (a chain's length halves, at least, with each round)
+        moved = false;
+        for (uint32_t li = threadIdx.x; li < here; li += kThreads) {
+            const int32_t up = p[li], r = p[up];
+            if (r != up) {
+                p[li] = r;
+                moved = true;
+            }
+        }
+        moved = __syncthreads_or(moved);
+    }
+    while (open) {
+        const int k = __ffsll((long long)open) - 1, i = k / D, mu = k - i * D;
+        open &= open - 1ull;
+        const uint32_t li = threadIdx.x + (uint32_t)(i * kThreads);
+        uint32_t lb[D], to = 0;
+        neighbours(li, lb);
+#pragma unroll
+        for (int m = 0; m < D; ++m)
+            if (m == mu) to = lb[m];
+        lunite(p, (int32_t)li, (int32_t)to, cap, a.ctrl);
+    }
+    __syncthreads();
+    for (uint32_t li = threadIdx.x; li < here; li += kThreads) {
+        const int32_t r = lfind(p, (int32_t)li, cap, a.ctrl);
+        const uint32_t s = s0 + li;
+        a.local_root[s] = (uint16_t)r;
+        if (r == (int32_t)li) a.parent[s] = (int32_t)s;
+        if (!KEYED) a.fresh[s] = r == (int32_t)li ? 1 : 0;  // root_rank_kernel's candidates
+    }
+}
 
 // Labels tile `tile`; the CTA may reuse `sm` at once.
-template <int D, bool SMALL, bool KEYED>
+template <int D, int SHAPE, bool KEYED>
 __device__ __forceinline__ void label_tile(const ClusterArgs &a, uint32_t sweep, uint32_t tile,
-                                           LabelShared<Tile<D, SMALL>> &sm) {
-    using T = Tile<D, SMALL>;
+                                           LabelShared<Tile<D, SHAPE>> &sm) {
+    using T = Tile<D, SHAPE>;
     constexpr int BY = T::BY, BZ = T::BZ, TX = T::TX, TY = T::TY, TZ = T::TZ, G = T::G;
     int32_t *p = sm.p;
     const T t(a.g);
@@ -708,10 +891,44 @@ __device__ __forceinline__ void label_tile(const ClusterArgs &a, uint32_t sweep,
     }
 }
 
-template <int D, bool SMALL, bool KEYED>
-__global__ void __launch_bounds__(kThreads, D == 2 && !SMALL ? 5 : 1) tile_hook_kernel(ClusterArgs a) {
-    __shared__ LabelShared<Tile<D, SMALL>> sm;
-    label_tile<D, SMALL, KEYED>(a, a.sweep32, blockIdx.x, sm);
+template <int D, int SHAPE, bool KEYED>
+__global__ void __launch_bounds__(kThreads, D == 2 && (SHAPE == kLarge || SHAPE == kNarrow) ? 5 : 1) tile_hook_kernel(ClusterArgs a) {
+    __shared__ LabelShared<Tile<D, SHAPE>> sm;
+    after_previous();
+    if constexpr (SHAPE == kFlat) label_flat<D, KEYED>(a, a.sweep32, blockIdx.x, sm.p);
+    else label_tile<D, SHAPE, KEYED>(a, a.sweep32, blockIdx.x, sm);
+}
+
+// unite_edges for tiles of consecutive sites: the bonds whose ends lie in two of them.
+template <int D, bool KEYED>
+__device__ __forceinline__ void unite_flat_edges(const ClusterArgs &a, uint32_t sweep) {
+    using T = Tile<D, kFlat>;
+    const T t(a.g);
+    const BondCut cut(a, sweep);
+    if (KEYED && !BondCut::some(a)) return;
+    const int64_t n = a.g.n_sites, stride = (int64_t)gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31;
+    for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); c0 < n; c0 += stride) {
+        const int64_t s = c0 + lane;
+        int32_t x[D];
+        site_coords<D>(a.g, s < n ? s : 0, x);
+#pragma unroll
+        for (int mu = 0; mu < D; ++mu) {
+            const int64_t nb = nbr_plus(a.g, s, x, mu);
+            int32_t pa = -1, pb = -1;
+            if (s < n && nb / T::kSites != s / T::kSites) {
+                const bool open = KEYED ? (a.state[s] == a.state[nb]) & cut.open((uint32_t)s * (uint32_t)D + (uint32_t)mu)
+                                        : (a.bonds[s] >> mu) & 1u;
+                if (open) {
+                    pa = (int32_t)t.local_root(a.local_root, (uint32_t)s, x);
+                    pb = (int32_t)t.local_root(a.local_root, (uint32_t)nb, x);
+                }
+            }
+            const int32_t qa = __shfl_up_sync(0xffffffffu, pa, 1), qb = __shfl_up_sync(0xffffffffu, pb, 1);
+            const bool repeat = lane > 0 && qa == pa && qb == pb;
+            if (pa >= 0 && !repeat) unite(a.parent, pa, pb, a.cap, a.ctrl);
+        }
+    }
 }
 
 // Global unions for the open bonds that leave their tile: of the tiles' last
@@ -719,9 +936,9 @@ __global__ void __launch_bounds__(kThreads, D == 2 && !SMALL ? 5 : 1) tile_hook_
 // index space), and every bond along the directions past the tile's.  A lane
 // whose ends' local roots are the lane before's leaves the union to that lane:
 // along a tile edge a large cluster meets another at many sites.
-template <int D, bool SMALL, bool KEYED>
+template <int D, int SHAPE, bool KEYED>
 __device__ __forceinline__ void unite_edges(const ClusterArgs &a, uint32_t sweep) {
-    using T = Tile<D, SMALL>;
+    using T = Tile<D, SHAPE>;
     const T t(a.g);
     const BondCut cut(a, sweep);
     const int64_t n = a.g.n_sites;
@@ -783,9 +1000,11 @@ __device__ __forceinline__ void unite_edges(const ClusterArgs &a, uint32_t sweep
     }
 }
 
-template <int D, bool SMALL, bool KEYED>
+template <int D, int SHAPE, bool KEYED>
 __global__ void __launch_bounds__(kThreads) boundary_hook_kernel(ClusterArgs a) {
-    unite_edges<D, SMALL, KEYED>(a, a.sweep32);
+    after_previous();
+    if constexpr (SHAPE == kFlat) unite_flat_edges<D, KEYED>(a, a.sweep32);
+    else unite_edges<D, SHAPE, KEYED>(a, a.sweep32);
 }
 
 // Read-only find for the passes after the unions: a compressing find could
@@ -892,10 +1111,10 @@ __device__ __forceinline__ void store_row(uint8_t *state, uint32_t s, int count,
 }
 
 // Every site's parent becomes its root (for the readers of labels and sizes).
-template <int D, bool SMALL>
+template <int D, int SHAPE>
 __global__ void __launch_bounds__(kThreads) flatten_kernel(ClusterArgs a) {
     // (the pass has stored each local root's root at the local root)
-    using T = Tile<D, SMALL>;
+    using T = Tile<D, SHAPE>;
     __shared__ RelabelShared<T> sm;
     tile_relabel<T>(
         a, blockIdx.x, sm, [](int32_t, int32_t) { return (uint8_t)0; },
@@ -907,11 +1126,12 @@ __global__ void __launch_bounds__(kThreads) flatten_kernel(ClusterArgs a) {
 }
 
 // keyed (cluster_relabel.wgsl:72-89), every cluster
-template <int D, bool SMALL>
+template <int D, int SHAPE>
 __global__ void __launch_bounds__(kThreads) relabel_keyed_kernel(ClusterArgs a) {
+    after_previous();
     const uint32_t q = (uint32_t)a.q;
     const bool forced = a.relabel == PLQ_RELABEL_FORCED;
-    using T = Tile<D, SMALL>;
+    using T = Tile<D, SHAPE>;
     __shared__ RelabelShared<T> sm;
     tile_relabel<T>(
         a, blockIdx.x, sm,
@@ -965,6 +1185,7 @@ __device__ __forceinline__ uint32_t fresh_label(const ClusterArgs &a, u128 st, u
 // also lists every such place of the stream (SecondDraws resolves them).
 template <int D>
 __global__ void __launch_bounds__(kThreads) root_rank_kernel(ClusterArgs a) {
+    after_previous();
     const int64_t n = a.g.n_sites;
     const int64_t chunk = take_chunk(a, true);
     if (chunk >= a.n_chunks) {
@@ -1057,11 +1278,12 @@ __device__ __noinline__ uint8_t moved_label(const ClusterArgs &a, int32_t root, 
 // stream: the labels to the sites, those behind a second draw drawn again (by every tile that
 // meets the cluster), and the position behind the second draws.  A sweep without one, nearly
 // every sweep, pays a load per CTA for it.
-template <int D, bool SMALL>
+template <int D, int SHAPE>
 __global__ void __launch_bounds__(kThreads, 8) apply_fresh_kernel(const __grid_constant__ ClusterArgs a) {
-    using T = Tile<D, SMALL>;
+    using T = Tile<D, SHAPE>;
     __shared__ RelabelShared<T> sm;
     __shared__ SecondDraws sd;
+    after_previous();
     const int listed = *a.event_count;
     if (listed) {
         if (threadIdx.x == 0) {
@@ -1244,10 +1466,10 @@ __device__ bool wolff_grow(const ClusterArgs &a, uint32_t sweep, uint32_t seed, 
     return begin == end;
 }
 
-template <int D, bool SMALL>
+template <int D, int SHAPE>
 __global__ void __launch_bounds__(kThreads, 4)
 wolff_kernel(ClusterArgs a, WolffSync *w, uint32_t n_tiles, unsigned long long launch) {
-    using T = Tile<D, SMALL>;
+    using T = Tile<D, SHAPE>;
     constexpr size_t kBytes = sizeof(LabelShared<T>) > sizeof(RelabelShared<T>)
                                   ? (sizeof(LabelShared<T>) > sizeof(GrowShared) ? sizeof(LabelShared<T>) : sizeof(GrowShared))
                                   : (sizeof(RelabelShared<T>) > sizeof(GrowShared) ? sizeof(RelabelShared<T>) : sizeof(GrowShared));
@@ -1317,7 +1539,8 @@ wolff_kernel(ClusterArgs a, WolffSync *w, uint32_t n_tiles, unsigned long long l
                 if (threadIdx.x == 0) s_stop = wolff_ended_by_growth(*small, id);
                 __syncthreads();
                 if (s_stop) break;
-                label_tile<D, SMALL, true>(a, sweep, tile, sm);
+                if constexpr (SHAPE == kFlat) label_flat<D, true>(a, sweep, tile, sm.p);
+                else label_tile<D, SHAPE, true>(a, sweep, tile, sm);
                 __syncthreads();
             }
         }
@@ -1325,7 +1548,8 @@ wolff_kernel(ClusterArgs a, WolffSync *w, uint32_t n_tiles, unsigned long long l
         if (threadIdx.x == 0) s_stop = wolff_ended_by_growth(*small, id);
         __syncthreads();
         if (s_stop) continue;
-        unite_edges<D, SMALL, true>(a, sweep);
+        if constexpr (SHAPE == kFlat) unite_flat_edges<D, true>(a, sweep);
+        else unite_edges<D, SHAPE, true>(a, sweep);
         wolff_barrier(w, a.ctrl);
         // the seed's cluster takes its new state
         if (threadIdx.x == 0) {
@@ -1424,7 +1648,7 @@ struct ClusterDev {
     unsigned long long *desc = nullptr;
     int64_t n_chunks = 0;
     int64_t n_tiles = 0;  // CTAs of the kernels that take a tile each
-    bool small_tiles = false;
+    TileShape shape = kSmall;
     int32_t *events = nullptr;
     int *event_count = nullptr;
     int32_t *sizes = nullptr;
@@ -1474,37 +1698,41 @@ ClusterArgs cluster_args(plq_chain *c) {
 }
 
 // The kernels of one tile size (a CTA per tile, and the boundary unions).
-template <int D, bool SMALL>
+template <int D, int SHAPE>
 struct TileKernels {
-    static void label(const ClusterArgs &a, bool keyed, unsigned tiles, unsigned blocks, cudaStream_t st) {
+    using T = Tile<D, SHAPE>;
+    // The launches it makes.
+    static unsigned label(const ClusterArgs &a, bool keyed, unsigned tiles, unsigned blocks, cudaStream_t st) {
+        const bool edges = SHAPE != kFlat || tiles > 1;
         if (keyed) {
-            tile_hook_kernel<D, SMALL, true><<<tiles, kThreads, 0, st>>>(a);
-            boundary_hook_kernel<D, SMALL, true><<<blocks, kThreads, 0, st>>>(a);
+            launch_next(tile_hook_kernel<D, SHAPE, true>, tiles, st, a);
+            if (edges) launch_next(boundary_hook_kernel<D, SHAPE, true>, blocks, st, a);
         } else {
-            tile_hook_kernel<D, SMALL, false><<<tiles, kThreads, 0, st>>>(a);
-            boundary_hook_kernel<D, SMALL, false><<<blocks, kThreads, 0, st>>>(a);
+            launch_next(tile_hook_kernel<D, SHAPE, false>, tiles, st, a);
+            if (edges) launch_next(boundary_hook_kernel<D, SHAPE, false>, blocks, st, a);
         }
+        return edges ? 2 : 1;
     }
     static void relabel_keyed(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
-        relabel_keyed_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
+        launch_next(relabel_keyed_kernel<D, SHAPE>, tiles, st, a);
     }
     static void apply_fresh(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
-        apply_fresh_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
+        launch_next(apply_fresh_kernel<D, SHAPE>, tiles, st, a);
     }
     static cudaError_t wolff(ClusterArgs a, WolffSync *w, uint32_t tiles, unsigned long long launch, unsigned grid,
                              cudaStream_t st) {
         void *params[] = {&a, &w, &tiles, &launch};
-        return cudaLaunchCooperativeKernel((const void *)wolff_kernel<D, SMALL>, dim3(grid), dim3(kThreads), params, 0, st);
+        return cudaLaunchCooperativeKernel((const void *)wolff_kernel<D, SHAPE>, dim3(grid), dim3(kThreads), params, 0, st);
     }
     // A CTA per tile and the growing one, as many as are resident together.
     static cudaError_t wolff_grid(int64_t tiles, int sm_count, unsigned &grid) {
         int per_sm = 0;
-        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wolff_kernel<D, SMALL>, kThreads, 0);
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wolff_kernel<D, SHAPE>, kThreads, 0);
         grid = (unsigned)std::min<int64_t>(tiles + 1, (int64_t)per_sm * sm_count);
         return e != cudaSuccess || grid >= 2 ? e : cudaErrorLaunchOutOfResources;
     }
     static void flatten(const ClusterArgs &a, unsigned tiles, cudaStream_t st) {
-        flatten_kernel<D, SMALL><<<tiles, kThreads, 0, st>>>(a);
+        flatten_kernel<D, SHAPE><<<tiles, kThreads, 0, st>>>(a);
     }
 };
 
@@ -1538,13 +1766,11 @@ int sweep_t(plq_chain *c, uint64_t sweeps) {
         if (stream) {
             // PCG stream: the bond draws sit at scanned positions, so they are made in one pass
             lookback(a);
-            bonds_kernel<D, true><<<(unsigned)cd->n_chunks, kThreads, 0, c->stream>>>(a);
-            K::label(a, false, (unsigned)cd->n_tiles, gs, c->stream);
-            c->launches += 3;
+            launch_next(bonds_kernel<D, true>, (unsigned)cd->n_chunks, c->stream, a);
+            c->launches += 1 + K::label(a, false, (unsigned)cd->n_tiles, gs, c->stream);
         } else {
             // keyed: each bond is a closed form of its index, evaluated where it is used
-            K::label(a, true, (unsigned)cd->n_tiles, gs, c->stream);
-            c->launches += 2;
+            c->launches += K::label(a, true, (unsigned)cd->n_tiles, gs, c->stream);
         }
         if (!stream) {
             K::relabel_keyed(a, (unsigned)cd->n_tiles, c->stream);
@@ -1552,7 +1778,7 @@ int sweep_t(plq_chain *c, uint64_t sweeps) {
         } else {
             lookback(a);
             // ranks, and the labels with no second draws known; the labels to the sites
-            root_rank_kernel<D><<<(unsigned)cd->n_chunks, kThreads, 0, c->stream>>>(a);
+            launch_next(root_rank_kernel<D>, (unsigned)cd->n_chunks, c->stream, a);
             K::apply_fresh(a, (unsigned)cd->n_tiles, c->stream);
             c->launches += 2;
         }
@@ -1565,10 +1791,24 @@ int sweep_t(plq_chain *c, uint64_t sweeps) {
     return PLQ_OK;
 }
 
+// f on the kernels of the chain's tiles.
+template <int D, class F>
+auto with_tiles(const plq_chain *c, F f) {
+    const TileShape shape = static_cast<ClusterDev *>(c->cl)->shape;
+    if constexpr (D >= 2) {
+        if (shape == kFlat) return f(TileKernels<D, kFlat>());
+        if (shape == kWide) return f(TileKernels<D, kWide>());
+        if (shape == kLarge) return f(TileKernels<D, kLarge>());
+    }
+    if constexpr (D == 2) {
+        if (shape == kNarrow) return f(TileKernels<D, kNarrow>());
+    }
+    return f(TileKernels<D, kSmall>());
+}
+
 template <int D>
 int sweep_d(plq_chain *c, uint64_t sweeps) {
-    return static_cast<ClusterDev *>(c->cl)->small_tiles ? sweep_t<D, TileKernels<D, true>>(c, sweeps)
-                                                        : sweep_t<D, TileKernels<D, D == 1>>(c, sweeps);
+    return with_tiles<D>(c, [&](auto k) { return sweep_t<D, decltype(k)>(c, sweeps); });
 }
 
 }  // namespace
@@ -1584,8 +1824,7 @@ int cluster_validate(const plq_chain_desc *d) {
 template <int D>
 static cudaError_t wolff_grid_d(plq_chain *c, unsigned &grid) {
     ClusterDev *cd = static_cast<ClusterDev *>(c->cl);
-    return cd->small_tiles ? TileKernels<D, true>::wolff_grid(cd->n_tiles, c->ctx->sm_count, grid)
-                           : TileKernels<D, D == 1>::wolff_grid(cd->n_tiles, c->ctx->sm_count, grid);
+    return with_tiles<D>(c, [&](auto k) { return decltype(k)::wolff_grid(cd->n_tiles, c->ctx->sm_count, grid); });
 }
 
 static cudaError_t wolff_grid(plq_chain *c, unsigned &grid) {
@@ -1625,15 +1864,19 @@ int cluster_create(plq_chain *c) {
     c->pass_cap = (c->desc.flags & PLQ_FLAG_TINY_PASS_CAP) ? 1 : std::min<int64_t>(n + 64, 1 << 30);
     cd->n_chunks = (n + kChunk - 1) / kChunk;
     size_t tile_sites = 0;
-    auto tiles = [&](auto large, auto small_t, bool is_large) {
-        cd->small_tiles = !is_large;
-        cd->n_tiles = is_large ? large.tiles(n) : small_t.tiles(n);
-        tile_sites = (size_t)cd->n_tiles * (is_large ? decltype(large)::kSites : decltype(small_t)::kSites);
+    auto tiles = [&](auto dims) {
+        constexpr int D = decltype(dims)::value;
+        cd->shape = tile_shape<D>(c->g, c->ctx->sm_count, c->desc.rng == PLQ_RNG_KEYED);
+        with_tiles<D>(c, [&](auto k) {
+            using T = typename decltype(k)::T;
+            cd->n_tiles = T(c->g).tiles(n);
+            tile_sites = (size_t)cd->n_tiles * T::kSites;
+        });
     };
     switch (c->d) {  // (d > 3 has the tiles of d = 3)
-        case 1: tiles(Tile<1, false>(c->g), Tile<1, true>(c->g), false); break;
-        case 2: tiles(Tile<2, false>(c->g), Tile<2, true>(c->g), large_tiles<2>(c->g, c->ctx->sm_count)); break;
-        default: tiles(Tile<3, false>(c->g), Tile<3, true>(c->g), large_tiles<3>(c->g, c->ctx->sm_count)); break;
+        case 1: tiles(std::integral_constant<int, 1>()); break;
+        case 2: tiles(std::integral_constant<int, 2>()); break;
+        default: tiles(std::integral_constant<int, 3>()); break;
     }
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void **p, size_t bytes) {
@@ -1698,8 +1941,7 @@ void cluster_free(plq_chain *c) {
 template <int D>
 static void flatten_d(plq_chain *c) {
     ClusterDev *cd = static_cast<ClusterDev *>(c->cl);
-    if (cd->small_tiles) TileKernels<D, true>::flatten(cluster_args(c), (unsigned)cd->n_tiles, c->stream);
-    else TileKernels<D, D == 1>::flatten(cluster_args(c), (unsigned)cd->n_tiles, c->stream);
+    with_tiles<D>(c, [&](auto k) { decltype(k)::flatten(cluster_args(c), (unsigned)cd->n_tiles, c->stream); });
 }
 
 static void flatten(plq_chain *c) {
