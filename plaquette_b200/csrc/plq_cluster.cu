@@ -41,6 +41,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 #include <vector>
@@ -1840,6 +1841,23 @@ static cudaError_t wolff_grid(plq_chain *c, unsigned &grid) {
     }
 }
 
+// The CTAs of a Wolff launch, of `most` that are resident together.  The launch is cooperative, and
+// launches of chains on other streams run beside it only while all of their CTAs fit: where
+// large clusters are rare, CTAs that wait to label them would keep other chains waiting
+// (eight hot chains, 3D Ising 128^3 at beta = 0.1 on eight streams: 21 us an update of each with
+// 513 CTAs, 2.8 with 33, 2.6 alone).  A bond whose ends are not connected otherwise is open with
+// probability t = p / (p + q (1 - p)), so on a tree generation k of a growth holds 2 d t ((2 d - 1) t)^(k - 1)
+// sites; that bounds how often a cluster outgrows the limit, and a label pass takes
+// about 8 us for each time the tiles exceed the CTAs: the CTAs keep that to 0.2 us an update, and
+// a pass to 16 tiles a CTA (a cold start's first clusters are large at any coupling).
+static unsigned wolff_ctas(unsigned most, int64_t n_tiles, int d, int q, double p) {
+    const double t = p / (p + q * (1 - p)), c = (2 * d - 1) * t;
+    if (!(c < 1)) return most;
+    const double outgrown = 2 * d * t * std::pow(c, grow_generations((uint32_t)n_tiles) - 1);
+    const double wanted = 1 + std::max(40 * outgrown, 1.0 / 16) * (double)n_tiles;
+    return wanted < most ? std::max(2u, (unsigned)wanted) : most;
+}
+
 int cluster_create(plq_chain *c) {
     ClusterDev *cd = new ClusterDev();
     c->cl = cd;
@@ -1886,6 +1904,7 @@ int cluster_create(plq_chain *c) {
         alloc((void **)&cd->wolff, sizeof(WolffSync));
         if (e == cudaSuccess) e = cudaMemsetAsync(cd->wolff, 0, sizeof(WolffSync), c->stream);
         if (e == cudaSuccess) e = wolff_grid(c, cd->wolff_grid);
+        if (e == cudaSuccess) cd->wolff_grid = wolff_ctas(cd->wolff_grid, cd->n_tiles, c->d, c->q, p);
         alloc((void **)&cd->parent, sizeof(int32_t) * (size_t)n);
         alloc((void **)&cd->local_root, sizeof(uint16_t) * tile_sites);
     } else {

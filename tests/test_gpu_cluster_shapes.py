@@ -2,7 +2,8 @@
 tile and one site more, short rows on flat and narrow tiles, few rows on wide and
 small ones, block tiles at 3D sizes one below, at and above theirs, extents of 1
 and 2 along any direction, both streams; states, labels and sizes are the
-oracle's."""
+oracle's.  Wolff on the few CTAs of a hot coupling, with the large first clusters
+of a cold start."""
 import numpy as np
 import pytest
 
@@ -65,6 +66,7 @@ def test_stream(oracle, gpu, shape):  # noqa: F811
 
 WOLFF = [(plq.ISING, 2, s, 1.1 * _beta(s)) for s in
          [(32, 32), (41, 25), (8, 4098), (33, 20000), (140000, 8), (65, 33, 31), (8, 200, 180), (300, 2, 2), (4, 5, 6, 20)]]
+WOLFF += [(plq.POTTS, 20, (200, 300), 0.9), (plq.POTTS, 20, (40, 40, 40), 0.5), (plq.ISING, 2, (40, 50, 60), 0.1)]
 
 
 @pytest.mark.parametrize("case", WOLFF, ids=lambda c: f"{c[0]}-{c[1]}-{'x'.join(map(str, c[2]))}")
