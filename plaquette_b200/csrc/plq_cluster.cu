@@ -352,7 +352,9 @@ __device__ __forceinline__ int32_t find_root(int32_t *parent, int32_t x, int cap
 // Unite the sets of a and b: the larger root is hooked under the smaller by an
 // atomic minimum on its parent.  Where that root was hooked in the meantime, its
 // parent becomes the smaller of the two all the same, and the link that gave way
-// (the old parent's) is united in turn: no attempt is repeated, so many lanes
+// (the old parent's) is united in turn, the reduction of Y. Komura, "GPU-based
+// cluster-labeling algorithm without the use of conventional iteration" (Comput.
+// Phys. Commun. 194, 2015): no attempt is repeated, so many lanes
 // hooking to one root do not wait for each other as they do on a CAS
 // (tile_hook_kernel on 2D Ising 4096^2 with 32-row blocks: 145 us with the CAS,
 // 131 with this).
@@ -469,7 +471,7 @@ struct Tile {  // block (per warp): 32 x BY x BZ; tile: WX x WY x WZ blocks
 // order, every bond between two of them is a bond of the tile, periodic ones too.
 template <int D>
 struct Tile<D, kFlat> {
-    static constexpr int TX = 2048, kSites = 2048, kDims = D;
+    static constexpr int TX = 2048, kSites = 2048;
 
     int32_t L[1];
     uint32_t n;
