@@ -56,7 +56,7 @@ enum plq_rng { PLQ_RNG_STREAM = 0, PLQ_RNG_KEYED = 1 };
  * against the other). */
 #define PLQ_FLAG_NO_FUSED 1
 /* Cap every cluster-labelling find and union at one step, so any real merge
- * trips the cap: exercises the PLQ_ECAP path (gpu_cluster.rs:512-518) on the
+ * that walks trips the cap: exercises the PLQ_ECAP path (gpu_cluster.rs:512-518) on the
  * host side without any device fault. */
 #define PLQ_FLAG_TINY_PASS_CAP 2
 /* Fused 3D sweep only: never issue the tile copies of one z-plane and wait

@@ -12,10 +12,10 @@
 //               exclusive scan (decoupled look-back) over agreeing bonds.
 //  2. labels -- lock-free union-find: every open bond unites its ends by
 //               hooking the larger root under the smaller (an atomic minimum), first
-//               inside 64x64 tiles in shared memory (tile_hook_kernel), then
+//               inside a tile in shared memory (tile_hook_kernel), then
 //               for the bonds that leave a tile (boundary_hook_kernel); the
-//               relabel pass walks each site to its root (a short walk: sites
-//               point at their tile-local roots) and stores it.  Roots only
+//               relabel pass walks each tile-local root to its cluster's root
+//               and hands that to the sites of the tile.  Roots only
 //               ever hook under smaller roots, so each component ends rooted
 //               at its minimum site: the canonical min-site label of the
 //               reference GPU (the fixed point of cluster_prelude.wgsl:113-147),
@@ -665,7 +665,8 @@ __device__ __forceinline__ void label_flat(const ClusterArgs &a, uint32_t sweep,
             if (((mine >> mu) & 1u) && lb[mu] > li && p[lb[mu]] == (int32_t)li) open &= ~(1ull << (i * D + mu));
     }
     __syncthreads();
-    for (bool moved = true; moved;) {  // (a chain's length halves, at least, with each round)
+    bool moved = true;
+    for (int round = 0; moved && round < 16; ++round) {  // (a chain's length halves, at least, with each)
         moved = false;
         for (uint32_t li = threadIdx.x; li < here; li += kThreads) {
             const int32_t up = p[li], r = p[up];

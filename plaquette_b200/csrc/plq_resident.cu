@@ -10,7 +10,7 @@
 // primaries.
 //
 // us a sweep, a launch per pass / resident, keyed: Ising 64^2 8.3 / 1.1, 48 x 40 x
-// 36 heat bath 8.2 / 3.4, 512^2 9.5 / 3.8, 100^3 12.3 / 6.7, 250^3 124 / 31; gauge 24^4
+// 36 heat bath 8.2 / 3.4, 512^2 9.5 / 3.8, 100^3 12.3 / 6.7, 250^3 124 / 28.5; gauge 24^4
 // 49 / 16.7, 48^3 37 / 12.6; Potts q = 3 64^3 heat bath 8.6 / 5.4, PCG stream 12.4 /
 // 10.1.  What is left of a small pass is one thread's chain of instructions (about
 // 0.55 us) and the barrier: a cluster's with the words' way through L2 0.7 us more, a
