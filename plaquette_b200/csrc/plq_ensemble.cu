@@ -1981,8 +1981,44 @@ cudaError_t job_repack(const ServerJob *j, bool unpack, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-// Allocate and upload a job's resident state (worker thread, device current).
-int job_admit(ServerJob *j, cudaStream_t stream) {
+// q = 2 and gauge jobs run packed while their rows find a place beside the bytes on which a job
+// is admitted: in what the budget leaves, and on the device.  False: the job runs on its bytes.
+bool job_pack(ServerJob *j, cudaStream_t stream) {
+    EnsMember &mem = j->mem;
+    const uint64_t bytes = packed_bytes(j->desc, mem.n_vars);
+    void *rows = nullptr;
+    cudaError_t e = cudaMalloc(&rows, bytes);
+    if (e == cudaSuccess) {
+        mem.pk = rows;
+        mem.pk_wide = j->desc.model != PLQ_GAUGE && j->desc.shape[0] > 32 ? 1 : 0;
+        e = job_repack(j, false, stream);
+    }
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        if (rows) cudaFree(rows);
+        mem.pk = nullptr;
+        return false;
+    }
+    mem.wpt = tuned_wpt(j->desc, true);
+    j->allocs.push_back(rows);
+    j->rows = bytes;
+    return true;
+}
+
+// An active job goes on on its bytes (between ticks); false: its rows stay.
+bool job_unpack(ServerJob *j, cudaStream_t stream) {
+    EnsMember &mem = j->mem;
+    if (job_repack(j, true, stream) != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess) return false;
+    j->allocs.erase(std::find(j->allocs.begin(), j->allocs.end(), mem.pk));
+    cudaFree(mem.pk);
+    mem.pk = nullptr;
+    mem.wpt = tuned_wpt(j->desc, false);
+    j->rows = 0;
+    return true;
+}
+
+// Allocate and upload a job's resident state (worker thread, device current); j->rows: its packed rows'.
+int job_admit(ServerJob *j, bool room_for_rows, cudaStream_t stream) {
     const plq_chain_desc &d = j->desc;
     EnsMember &mem = j->mem;
     std::memset(&mem, 0, sizeof mem);
@@ -2085,48 +2121,13 @@ int job_admit(ServerJob *j, cudaStream_t stream) {
     j->ts.hb24 = (const uint32_t *)up(t.hb24.data(), t.hb24.size() * 4);
     j->ts.metro53 = (const uint64_t *)up(t.metro53.data(), t.metro53.size() * 8);
     j->ts.metro24 = (const uint32_t *)up(t.metro24.data(), t.metro24.size() * 4);
+    if (e == cudaSuccess && room_for_rows) (void)job_pack(j, stream);  // (without a place: on its bytes)
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) {
         job_release(j);
         return plq_fail(e == cudaErrorMemoryAllocation ? PLQ_ENOMEM : PLQ_ECUDA, cudaGetErrorString(e));
     }
     return PLQ_OK;
-}
-
-// q = 2 and gauge jobs run packed while their rows find a place beside the bytes on which a job
-// is admitted: in what the budget leaves, and on the device.  False: the job runs on its bytes.
-bool job_pack(ServerJob *j, cudaStream_t stream) {
-    EnsMember &mem = j->mem;
-    const uint64_t bytes = packed_bytes(j->desc, mem.n_vars);
-    void *rows = nullptr;
-    cudaError_t e = cudaMalloc(&rows, bytes);
-    if (e == cudaSuccess) {
-        mem.pk = rows;
-        mem.pk_wide = j->desc.model != PLQ_GAUGE && j->desc.shape[0] > 32 ? 1 : 0;
-        e = job_repack(j, false, stream);
-    }
-    if (e != cudaSuccess) {
-        (void)cudaGetLastError();
-        if (rows) cudaFree(rows);
-        mem.pk = nullptr;
-        return false;
-    }
-    mem.wpt = tuned_wpt(j->desc, true);
-    j->allocs.push_back(rows);
-    j->rows = bytes;
-    return true;
-}
-
-// An active job goes on on its bytes (between ticks); false: its rows stay.
-bool job_unpack(ServerJob *j, cudaStream_t stream) {
-    EnsMember &mem = j->mem;
-    if (job_repack(j, true, stream) != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess) return false;
-    j->allocs.erase(std::find(j->allocs.begin(), j->allocs.end(), mem.pk));
-    cudaFree(mem.pk);
-    mem.pk = nullptr;
-    mem.wpt = tuned_wpt(j->desc, false);
-    j->rows = 0;
-    return true;
 }
 
 // Device buffers of one tick's launch; grown, never shrunk.
@@ -2342,20 +2343,12 @@ void worker_loop(plq_server *S) {
             S->rows -= rows;
         }
         for (ServerJob *j : admit) {
-            int rc = job_admit(j, stream);
-            if (rc == PLQ_OK && packed_eligible(j->desc)) {
-                const uint64_t rows = packed_bytes(j->desc, j->mem.n_vars);
-                bool room;
-                {
-                    std::lock_guard<std::mutex> lock(S->mu);
-                    room = S->used + S->rows + rows <= S->budget;
-                    if (room) S->rows += rows;
-                }
-                if (room && !job_pack(j, stream)) {
-                    std::lock_guard<std::mutex> lock(S->mu);
-                    S->rows -= rows;
-                }
+            bool room = false;
+            if (packed_eligible(j->desc)) {
+                std::lock_guard<std::mutex> lock(S->mu);
+                room = S->used + S->rows + packed_bytes(j->desc, desc_vars(j->desc)) <= S->budget;
             }
+            int rc = job_admit(j, room, stream);
             std::lock_guard<std::mutex> lock(S->mu);
             if (rc != PLQ_OK) {
                 S->used -= j->footprint;
@@ -2365,6 +2358,7 @@ void worker_loop(plq_server *S) {
                 j->t_finish = now_s();
                 S->cv_done.notify_all();
             } else {
+                S->rows += j->rows;
                 j->state = PLQ_JOB_ACTIVE;
                 j->t_admit = now_s();
                 S->active.push_back(j);
