@@ -97,7 +97,10 @@ extern "C" int plq_ctx_create(int device_ordinal, plq_ctx **out) {
     return PLQ_OK;
 }
 
-extern "C" void plq_ctx_destroy(plq_ctx *ctx) { delete ctx; }
+extern "C" void plq_ctx_destroy(plq_ctx *ctx) {
+    if (ctx) plq_readback_release(ctx->device);  // (a program may reset the device between contexts)
+    delete ctx;
+}
 
 // ------------------------------------------------------------ helpers
 extern "C" uint32_t plq_fold_seed(uint64_t seed) { return (uint32_t)(seed ^ (seed >> 32)); }

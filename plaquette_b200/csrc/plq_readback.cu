@@ -24,7 +24,7 @@ namespace {
 
 constexpr size_t kPiece = size_t(1) << 20;
 constexpr int kWorkers = 8;
-constexpr size_t kKept = 2;  // sets kept for later calls (8 MiB of pinned memory each)
+constexpr size_t kKept = 2;  // sets kept for later calls (8 MiB of pinned memory each) until a context ends
 
 // A set of pinned buffers and their events, one a worker; used by one call at a time.
 struct Staging {
@@ -80,6 +80,22 @@ void give_back(Staging *s) {
 }
 
 }  // namespace
+
+void plq_readback_release(int device) {
+    for (;;) {
+        Staging *s = nullptr;
+        {
+            std::lock_guard<std::mutex> lock(g_mutex);
+            for (size_t k = 0; k < g_idle.size() && !s; ++k)
+                if (g_idle[k]->device == device) {
+                    s = g_idle[k];
+                    g_idle.erase(g_idle.begin() + (long)k);
+                }
+        }
+        if (!s) return;
+        destroy(s);
+    }
+}
 
 cudaError_t plq_readback(void *dst, const void *src, size_t bytes, int device, cudaStream_t stream) {
     cudaPointerAttributes attr;

@@ -10,3 +10,5 @@
 // stream as cudaMemcpyAsync queues it.
 constexpr size_t kReadbackStaged = size_t(32) << 20;
 cudaError_t plq_readback(void *dst, const void *src, size_t bytes, int device, cudaStream_t stream);
+// Gives back the pinned buffers that earlier copies from `device` left for later ones.
+void plq_readback_release(int device);
