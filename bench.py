@@ -292,9 +292,9 @@ def measure_local(name, steps, warmup, ctx, e2e=True):
                    "(537 MB, larger than L2) from HBM once per sweep")
     passes = max(1, steps * per_sweep)  # launches of the dominant kernel
     if resident:
-        # every sweep of the timed call in one launch, on words of one bit a site
+        # many sweeps a launch, on words of one bit a site
         kernel, passes = "stream_kernel" if w[3] == "stream" else "resident_kernel", launches
-        l2_note = ("134 MB byte state read (packed) and written (unpacked) once per advance call; the sweeps run "
+        l2_note = ("134 MB byte state read (packed) and written (unpacked) once per launch of 64 sweeps, which run "
                    "on a 16.8 MB bit-packed copy that stays in L2")
     per_launch_ms = dev_ms / passes
     alg_bytes = BYTES_PER_UPDATE * N_SITES * steps // passes  # per launch of the dominant kernel

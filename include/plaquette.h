@@ -204,9 +204,9 @@ int plq_chain_cluster_histogram(plq_chain *chain, int64_t *hist, int32_t nbins);
  * "lookback" (stream Metropolis, whose draws' places depend on the states),
  * "cluster". */
 const char *plq_chain_path(plq_chain *chain);
-/* 1 if the sweeps of a call run in one launch with a barrier per pass (q = 2
- * chains on packed words then, whatever plq_chain_path names), 0 if each pass
- * is a launch. */
+/* 1 if the sweeps of a call run in one launch (or few, of at most 2^33 updates)
+ * with a barrier per pass (q = 2 chains on packed words then, whatever
+ * plq_chain_path names), 0 if each pass is a launch. */
 int plq_chain_resident(plq_chain *chain);
 /* Kernels this chain has launched so far. */
 uint64_t plq_chain_launches(plq_chain *chain);

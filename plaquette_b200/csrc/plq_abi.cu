@@ -710,7 +710,7 @@ static int fused_sweep(plq_chain *c) {
 
 // `samples` times `sweeps` sweeps in one launch, each followed by a snapshot
 // and a measurement where there is a place for them.
-static int resident_sweeps(plq_chain *c, uint64_t samples, uint64_t sweeps, uint8_t *snapshots, long long *primaries) {
+static int resident_launch(plq_chain *c, uint64_t samples, uint64_t sweeps, uint8_t *snapshots, long long *primaries) {
     if (!samples || (!sweeps && !snapshots && !primaries)) return PLQ_OK;
     ResidentArgs r;
     std::memset(&r, 0, sizeof r);
@@ -737,6 +737,28 @@ static int resident_sweeps(plq_chain *c, uint64_t samples, uint64_t sweeps, uint
     c->launches++;
     if (c->desc.rng == PLQ_RNG_STREAM && !c->lookback) c->host_pos += samples * sweeps * (uint64_t)c->n_vars;
     c->sweeps_done += samples * sweeps;
+    return PLQ_OK;
+}
+
+// The same in launches of at most 2^33 updates, some 20 ms of a lattice that fills the chip: a call of
+// any length leaves other streams' work its turns, as passes of their own did.  (512^3 on the PCG
+// stream, the dearest to pack and unpack: 0.1 ms of each 24.)
+static int resident_sweeps(plq_chain *c, uint64_t samples, uint64_t sweeps, uint8_t *snapshots, long long *primaries) {
+    const uint64_t most = std::max<uint64_t>(1, (uint64_t(1) << 33) / (uint64_t)c->n_vars);
+    const int np = primaries_count(c->desc.model, c->q);
+    while (samples) {
+        uint64_t last = sweeps;  // of a sample's sweeps, those in the launch that takes it
+        for (; last > most; last -= most) {
+            int rc = resident_launch(c, 1, most, nullptr, nullptr);
+            if (rc != PLQ_OK) return rc;
+        }
+        const uint64_t k = last < sweeps ? 1 : std::min(samples, std::max<uint64_t>(1, most / std::max<uint64_t>(1, sweeps)));
+        int rc = resident_launch(c, k, last, snapshots, primaries);
+        if (rc != PLQ_OK) return rc;
+        if (snapshots) snapshots += k * (uint64_t)c->n_vars;
+        if (primaries) primaries += k * (uint64_t)np;
+        samples -= k;
+    }
     return PLQ_OK;
 }
 

@@ -1749,7 +1749,8 @@ int sweep_t(plq_chain *c, uint64_t sweeps) {
     if (c->desc.extent == PLQ_EXTENT_SEEDED) {
         for (uint64_t left = sweeps; left;) {
             ClusterArgs a = cluster_args(c);
-            a.updates = std::min<uint64_t>(left, 1u << 30);
+            // (launches of some 20 ms, between which other streams' work takes its turn)
+            a.updates = std::min<uint64_t>(left, 1024);
             const cudaError_t e = K::wolff(a, cd->wolff, (uint32_t)cd->n_tiles, ++cd->wolff_launches, cd->wolff_grid,
                                            c->stream);
             c->launches++;
